@@ -210,6 +210,31 @@ __device__ __forceinline__ double divI(double x, double y) {
 }
 __device__ __forceinline__ float divI(float x, float y) { return x / y; }
 
+// (float)((double)c - (double)a * (double)b) for floats, on the FP32 pipes.  The product
+// is exact in double (48 bits), so the value is c - a*b rounded to 53 bits and then to 24;
+// one fma rounds it to 24 directly, the same unless the 53-bit value is the midpoint of
+// two floats.  The distance x - r of the exact value from the fma's result r is formed
+// from the product's and the sum's error terms (fma residual, Knuth's two-sum) to well
+// below 2^-18 of half an ulp; results within that of a midpoint (and r a power of two,
+// whose lower neighbour is closer, and tiny r) take the double expression out of line.
+// The three conversions to double, the product, the difference and the conversion back
+// ran on the FP64 unit and were most of the FP32 flux kernel: KH 2048^2 550 us a launch,
+// 163 us with this form (the rest of it: loads at the HBM rate).
+static __device__ __noinline__ float subProductNative(float c, float a, float b) {
+    return (float)((double)c - (double)a * (double)b);
+}
+__device__ __forceinline__ float subProduct(float c, float a, float b) {
+    const float r = fmaf(-a, b, c);
+    const float p = __fmul_rn(a, b), pe = fmaf(a, b, -p);                    // a*b = p + pe
+    const float s = __fsub_rn(c, p), v = __fsub_rn(s, c);
+    const float t = __fsub_rn(__fsub_rn(c, __fsub_rn(s, v)), __fadd_rn(p, v));   // c - p = s + t
+    const float e = __fsub_rn(__fadd_rn(__fsub_rn(s, r), t), pe);
+    const unsigned rb = __float_as_uint(r);
+    const float half = __uint_as_float(rb & 0x7F800000u) * 0x1p-24f;         // half an ulp of r
+    const bool near = fabsf(fabsf(e) - half) < 0x1p-18f * (half + fabsf(pe) + fabsf(t));
+    const bool edge = (rb << 1) != 0 && ((rb << 9) == 0 || (rb & 0x7FFFFFFFu) < 0x12800000u);   // |r| < 2^-90
+    return near || edge ? subProductNative(c, a, b) : r;
+}
 
 
 }  // namespace hgpu

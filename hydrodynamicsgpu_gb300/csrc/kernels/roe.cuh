@@ -304,7 +304,7 @@ __device__ __forceinline__ void roeFlux(const real* rec, const real* sL, const r
     const int N = D + 2;
     real avg[5], ft[5];
 #pragma unroll
-    for (int i = 0; i < N; ++i) avg[i] = (real)halfOf((double)(sR[i] + sL[i]));    // .5 * (stateR + stateL)
+    for (int i = 0; i < N; ++i) avg[i] = halfOf(sR[i] + sL[i]);    // .5 * (stateR + stateL)
     leftTransform<real, D, SIDE>(rec, avg, ft);
     // waves 1..N-2 share the eigenvalue vx: their epsilon and theta are the same values
     const real vx = rec[R_::VX];
@@ -338,7 +338,9 @@ __device__ __forceinline__ void roeFlux(const real* rec, const real* sL, const r
                 tape[((long long)FT_F * N + i) * V] = ft[i];
             }
         }
-        else ft[i] -= .5 * deltaFluxTilde * (theta + phi * epsMinusTheta);   // double literal: FP32 promotes
+        // FP32: the reference's double literal (.5 * ...) promotes the product and the
+        // difference; subProduct gives that value without the FP64 unit
+        else ft[i] = subProduct(ft[i], deltaFluxTilde, halfOf(theta + phi * epsMinusTheta));
     }
     rightTransform<real, D, SIDE>(rec, ft, F);
 }
