@@ -24,6 +24,7 @@ RoeAdjoint::RoeAdjoint(const ResolvedConfig& rc, cudaStream_t stream) : rc_(rc),
     for (int i = 0; i < 3; ++i) {
         ph_.dx[i] = rc.dx[i];
         ph_.rdx[i] = 1. / ph_.dx[i];
+        hostDivisor(ph_.dx[i], ph_.dxDiv[i]);
         for (int m = 0; m < 2; ++m) methods_[i][m] = i < rc.dim ? rc.cfg.boundary[i][m] : -1;
     }
     ph_.gamma = rc.gamma;

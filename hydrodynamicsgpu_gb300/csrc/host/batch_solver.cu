@@ -53,6 +53,7 @@ BatchSolver<real>::BatchSolver(const std::vector<hgpu_config>& cfgs) {
         for (int i = 0; i < 3; ++i) {
             p.ph.dx[i] = (real)r.dx[i];
             p.ph.rdx[i] = (real)1 / p.ph.dx[i];
+            hostDivisor(p.ph.dx[i], p.ph.dxDiv[i]);
         }
         p.ph.gamma = (real)r.gamma;
         p.ph.cfl = r.cfg.cfl;

@@ -442,6 +442,7 @@ Solver<real>::Solver(const ResolvedConfig& rc_) : rc(rc_) {
     for (int i = 0; i < 3; ++i) {
         ph.dx[i] = (real)rc.dx[i];
         ph.rdx[i] = (real)1 / ph.dx[i];
+        hostDivisor(ph.dx[i], ph.dxDiv[i]);
     }
     ph.gamma = (real)rc.gamma;
     ph.cfl = rc.cfg.cfl;

@@ -7,6 +7,7 @@
 // instructions, or a shorter FP64 sequence, wherever that is exact, and the plain
 // operation otherwise.  The float overloads are the plain operations.
 #pragma once
+#include <cstring>
 #include <cuda_runtime.h>
 
 namespace hgpu {
@@ -134,25 +135,6 @@ __device__ __forceinline__ double mulI(double x, double y) {
 }
 __device__ __forceinline__ float mulI(float x, float y) { return x * y; }
 
-// x / b given rb = RN(1/b) (b and rb normal): Markstein's quotient correction,
-//   q = RN(x*rb), r = x - b*q (exact, by fma), q' = RN(q + r*rb) = RN(x/b)
-// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Dev. 34(1), 1990; checked here against the hardware
-// division on 3.8e9 random and near-midpoint operand pairs, none differing).
-// A zero x over a finite nonzero b gives the zero of sign(x) xor sign(b); operands
-// outside a safe exponent window (zero, subnormal, huge, Inf, NaN -- so 0/0 and x/0
-// too) take the hardware division, so q' and r never leave the normal range.
-__device__ __forceinline__ double divByRecip(double x, double b, double rb) {
-    long long bx = bitsOf(x), bb = bitsOf(b);
-    int ex = (int)((bx >> 52) & 0x7FF), eb = (int)((bb >> 52) & 0x7FF);
-    if (isZeroBits(x) && eb != 0 && eb != 0x7FF) return fromBits((bx ^ bb) & (long long)0x8000000000000000ULL);
-    if (ex < 623 || ex > 1423 || eb < 623 || eb > 1423) return x / b;
-    double q = mulI(x, rb);
-    double r = fma(-b, q, x);
-    return fma(r, rb, q);
-}
-__device__ __forceinline__ float divByRecip(float x, float b, float rb) { return x / b; }
-
 static __device__ __noinline__ double divNative(double x, double y) { return x / y; }
 
 // 2^64 / d for the significand d in [1, 2) of y (its words given; y normal), from below
@@ -225,6 +207,39 @@ __device__ __forceinline__ double divI(double x, double y) {
     return quotientBits(xh, xl, yh, yl, recipBits(yh, yl));
 }
 __device__ __forceinline__ float divI(float x, float y) { return x / y; }
+
+// A divisor used by several quotients (a density, the cell size, an HLLC denominator):
+// its reciprocal bits are formed once, on the host for a constant, and a quotient then
+// costs about a product.  v is 0 where b is not normal.
+template <typename real> struct Divisor { real b; };
+template <> struct Divisor<double> { double b; unsigned long long v; };
+
+__device__ __forceinline__ Divisor<float> divisorOf(float b) { return {b}; }
+__device__ __forceinline__ Divisor<double> divisorOf(double b) {
+    const unsigned h = (unsigned)__double2hiint(b);
+    return {b, (h & 0x7FF00000u) - 0x00100000u < 0x7FE00000u ? recipBits(h, (unsigned)__double2loint(b)) : 0ull};
+}
+inline void hostDivisor(float b, Divisor<float>& d) { d.b = b; }
+inline void hostDivisor(double b, Divisor<double>& d) {
+    unsigned long long u;
+    memcpy(&u, &b, 8);
+    const unsigned long long m = (u & 0xFFFFFFFFFFFFFull) | (1ull << 52), e = (u >> 52) & 0x7FF;
+    d.b = b;
+    d.v = e - 1 >= 2046 ? 0ull : m == (1ull << 52) ? ~0ull : (unsigned long long)(((unsigned __int128)1 << 116) / m);
+}
+
+// x / d.b, the IEEE quotient (as divI)
+__device__ __forceinline__ float quotBy(float x, const Divisor<float>& d) { return x / d.b; }
+__device__ __forceinline__ double quotBy(double x, const Divisor<double>& d) {
+    const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
+    const unsigned yh = (unsigned)__double2hiint(d.b), yl = (unsigned)__double2loint(d.b);
+    const unsigned ex = xh & 0x7FF00000u, ey = yh & 0x7FF00000u;
+    if (ex - 0x00100000u >= 0x7FE00000u || d.v == 0 || ex - ey + (1021u << 20) >= (2044u << 20)) {
+        if (((xh << 1) | xl) == 0 && d.v != 0) return __hiloint2double((int)((xh ^ yh) & 0x80000000u), 0);
+        return divNative(x, d.b);
+    }
+    return quotientBits(xh, xl, yh, yl, d.v);
+}
 
 // (float)((double)c - (double)a * (double)b) for floats, on the FP32 pipes.  The product
 // is exact in double (48 bits), so the value is c - a*b rounded to 53 bits and then to 24;

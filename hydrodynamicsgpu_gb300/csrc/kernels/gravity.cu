@@ -61,18 +61,6 @@ __global__ void __launch_bounds__(kThreads) relaxRhsKernel(Grid g, GravityConst<
     rhs[c] = mulI(gc.fourPiG, (double)state[(long long)(D + 2) * c]);
 }
 
-// x / dx^2 of the relaxation, exact: FP64 by the quotient correction on RN(1 / dx^2)
-// (fp64ops.cuh divByRecip: two FMAs on the FP64 unit) or on the integer pipes (divI);
-// FP32 the float division.  Measured on GB300 (2048^2 sweep): the x neighbours by the
-// correction and the rest on the integer pipes balance the two units best (0.134 ms a
-// sweep; all on the integer pipes 0.168, every neighbour by the correction 0.154).
-template <bool RECIP>
-__device__ __forceinline__ double overDxSq(double x, double d, double rd) {
-    return RECIP ? divByRecip(x, d, rd) : divI(x, d);
-}
-template <bool RECIP>
-__device__ __forceinline__ float overDxSq(float x, float d, double) { return x / d; }
-
 // one colour of a relaxation sweep: blockIdx.y (+ gridDim.y * blockIdx.z) = the interior
 // row (y, z), thread x = the k-th cell of that colour along the row
 template <typename real, int D>
@@ -86,20 +74,20 @@ __global__ void __launch_bounds__(kThreads) relaxKernel(Grid g, GravityConst<rea
     const long long c = x + (long long)g.S[0] * (y + (long long)g.S[1] * z);
     // skewSum: +x, -x, +y, -y, +z, -z neighbours inside [2, S-3] (SelfGravitation.cl:39-51)
     real skewSum = (real)0;
-    if (x < g.S[0] - 3) skewSum = skewSum + overDxSq<true>(pot[c + 1], gc.dxSq[0], gc.rdxSq[0]);
-    if (x > 2) skewSum = skewSum + overDxSq<true>(pot[c - 1], gc.dxSq[0], gc.rdxSq[0]);
+    if (x < g.S[0] - 3) skewSum = skewSum + quotBy(pot[c + 1], gc.dxSq[0]);
+    if (x > 2) skewSum = skewSum + quotBy(pot[c - 1], gc.dxSq[0]);
     if (D > 1) {
         const long long sy = g.step[1];
-        if (y < g.S[1] - 3) skewSum = skewSum + overDxSq<false>(pot[c + sy], gc.dxSq[1], gc.rdxSq[1]);
-        if (y > 2) skewSum = skewSum + overDxSq<false>(pot[c - sy], gc.dxSq[1], gc.rdxSq[1]);
+        if (y < g.S[1] - 3) skewSum = skewSum + quotBy(pot[c + sy], gc.dxSq[1]);
+        if (y > 2) skewSum = skewSum + quotBy(pot[c - sy], gc.dxSq[1]);
     }
     if (D > 2) {
         const long long sz = g.step[2];
-        if (z < g.S[2] - 3) skewSum = skewSum + overDxSq<false>(pot[c + sz], gc.dxSq[2], gc.rdxSq[2]);
-        if (z > 2) skewSum = skewSum + overDxSq<false>(pot[c - sz], gc.dxSq[2], gc.rdxSq[2]);
+        if (z < g.S[2] - 3) skewSum = skewSum + quotBy(pot[c + sz], gc.dxSq[2]);
+        if (z > 2) skewSum = skewSum + quotBy(pot[c - sz], gc.dxSq[2]);
     }
     // (4. * M_PI * G * density - skewSum) / diag, in double for both precisions
-    pot[c] = (real)divI(rhs[c] - (double)skewSum, gc.diag);
+    pot[c] = (real)quotBy(rhs[c] - (double)skewSum, gc.diag);
 }
 
 // calcGravityDeriv of one cell into d (zero outside the interior), then the combine
@@ -125,7 +113,7 @@ __global__ void __launch_bounds__(kThreads) gravityCombineKernel(Grid g, Gravity
             const long long sp = g.step[side];
             const real dphi = pot[c + sp] - pot[c - sp];
             // (phi[next] - phi[prev]) / (2. * dx[side]): a double quotient, stored as real
-            const real gradient = (real)divI((double)dphi, gc.twoDx[side]);
+            const real gradient = (real)quotBy((double)dphi, gc.twoDx[side]);
             const real gravity = -gradient;
             const real f = mulI(density, gravity);
             d[1 + side] = zfix(-f);                                  // deriv (+0) -= density * gravity
@@ -148,13 +136,12 @@ GravityConst<real> gravityConst(const double dx[3], double G, int dim) {
     for (int i = 0; i < dim; ++i) {
         const real dxr = (real)dx[i];
         const real sq = dxr * dxr;                                  // DX * DX in the program's type
-        gc.dxSq[i] = sq;
-        gc.rdxSq[i] = 1. / (double)sq;                                // RN(1 / dx^2) for the exact quotient
+        hostDivisor(sq, gc.dxSq[i]);
         invSum = i == 0 ? 1. / (double)sq : invSum + 1. / (double)sq;
-        gc.twoDx[i] = 2. * (double)dxr;
+        hostDivisor(2. * (double)dxr, gc.twoDx[i]);
     }
-    for (int i = dim; i < 3; ++i) { gc.dxSq[i] = (real)1; gc.rdxSq[i] = 1.; gc.twoDx[i] = 2.; }
-    gc.diag = (double)(real)(-2. * invSum);                          // `const real diag`
+    for (int i = dim; i < 3; ++i) { hostDivisor((real)1, gc.dxSq[i]); hostDivisor(2., gc.twoDx[i]); }
+    hostDivisor((double)(real)(-2. * invSum), gc.diag);              // `const real diag`
     return gc;
 }
 

@@ -8,10 +8,9 @@ namespace hgpu {
 template <typename real>
 struct GravityConst {
     double fourPiG;   // 4. * M_PI * ((real)G), double
-    double diag;      // (double)(real)(-2. * (1. / (DX * DX) + ...)), `const real diag`
-    real dxSq[3];     // DX * DX in the program's type
-    double rdxSq[3];  // RN(1 / (DX * DX)), FP64 quotient correction
-    double twoDx[3];  // 2. * dx[side], double
+    Divisor<double> diag;      // (double)(real)(-2. * (1. / (DX * DX) + ...)), `const real diag`
+    Divisor<real> dxSq[3];     // DX * DX in the program's type
+    Divisor<double> twoDx[3];  // 2. * dx[side], double
 };
 
 template <typename real>

@@ -40,10 +40,10 @@ template <typename real, int D, bool GRAV = false>
 __device__ __forceinline__ void primitives(const real* st, real gamma, Prim<real, D>& p, real phi = (real)0) {
     const int E = D + 1;
     p.density = st[0];
-    p.invDensity = (real)divI(1., (double)p.density);
-    // VELOCITY: m/rho, by the correction step on RN(1/rho) in FP64 (fp64ops.cuh)
+    const Divisor<real> byRho = divisorOf(p.density);
+    p.invDensity = quotBy((real)1, byRho);   // FP32: the double quotient rounded to float is the float quotient
 #pragma unroll
-    for (int k = 0; k < D; ++k) p.v[k] = divByRecip(st[1 + k], p.density, p.invDensity);
+    for (int k = 0; k < D; ++k) p.v[k] = quotBy(st[1 + k], byRho);
     p.energyTotal = mulI(st[E], p.invDensity);
     p.potential = phi;
     primitivesFromVelocity<real, D, GRAV>(gamma, p);
@@ -248,22 +248,22 @@ __device__ __forceinline__ bool hllcFaceFromPrim(const Grid& g, const real* stL,
     } else if (leZero(sl) && geZero(sStar)) {
         real pressureLR = halfOf(L.pressure + R.pressure + mulI(mulI(L.density, sl - L.v[0]), sStar - L.v[0]) +
                                  mulI(mulI(R.density, sr - R.v[0]), sStar - R.v[0]));
-        // every component divides by (sl - sStar): one reciprocal, then exact corrected quotients
-        real den = sl - sStar, rden = divI((real)1., den);
-        flux[0] = divByRecip(mulI(sStar, mulI(sl, stL[0]) - fL[0]), den, rden);
-        flux[1] = divByRecip(mulI(sStar, mulI(sl, stL[1]) - fL[1]) + mulI(sl, pressureLR), den, rden);
+        // every component divides by (sl - sStar)
+        const Divisor<real> den = divisorOf(sl - sStar);
+        flux[0] = quotBy(mulI(sStar, mulI(sl, stL[0]) - fL[0]), den);
+        flux[1] = quotBy(mulI(sStar, mulI(sl, stL[1]) - fL[1]) + mulI(sl, pressureLR), den);
 #pragma unroll
-        for (int k = 1; k < D; ++k) flux[1 + k] = divByRecip(mulI(sStar, mulI(sl, stL[1 + k]) - fL[1 + k]), den, rden);
-        flux[E] = divByRecip(mulI(sStar, mulI(sl, stL[E]) - fL[E]) + mulI(mulI(sl, pressureLR), sStar), den, rden);
+        for (int k = 1; k < D; ++k) flux[1 + k] = quotBy(mulI(sStar, mulI(sl, stL[1 + k]) - fL[1 + k]), den);
+        flux[E] = quotBy(mulI(sStar, mulI(sl, stL[E]) - fL[E]) + mulI(mulI(sl, pressureLR), sStar), den);
     } else if (leZero(sStar) && geZero(sr)) {
         real pressureLR = halfOf(L.pressure + R.pressure + mulI(mulI(L.density, sl - L.v[0]), sStar - L.v[0]) +
                                  mulI(mulI(R.density, sr - R.v[0]), sStar - R.v[0]));
-        real den = sr - sStar, rden = divI((real)1., den);
-        flux[0] = divByRecip(mulI(sStar, mulI(sr, stR[0]) - fR[0]), den, rden);
-        flux[1] = divByRecip(mulI(sStar, mulI(sr, stR[1]) - fR[1]) + mulI(sr, pressureLR), den, rden);
+        const Divisor<real> den = divisorOf(sr - sStar);
+        flux[0] = quotBy(mulI(sStar, mulI(sr, stR[0]) - fR[0]), den);
+        flux[1] = quotBy(mulI(sStar, mulI(sr, stR[1]) - fR[1]) + mulI(sr, pressureLR), den);
 #pragma unroll
-        for (int k = 1; k < D; ++k) flux[1 + k] = divByRecip(mulI(sStar, mulI(sr, stR[1 + k]) - fR[1 + k]), den, rden);
-        flux[E] = divByRecip(mulI(sStar, mulI(sr, stR[E]) - fR[E]) + mulI(mulI(sr, pressureLR), sStar), den, rden);
+        for (int k = 1; k < D; ++k) flux[1 + k] = quotBy(mulI(sStar, mulI(sr, stR[1 + k]) - fR[1 + k]), den);
+        flux[E] = quotBy(mulI(sStar, mulI(sr, stR[E]) - fR[E]) + mulI(mulI(sr, pressureLR), sStar), den);
     } else if (leZero(sr)) {
 #pragma unroll
         for (int i = 0; i < N; ++i) flux[i] = fR[i];

@@ -266,6 +266,7 @@ void launchCfl(const ResolvedConfig& rc, int hllc, const void* state, long long 
     for (int i = 0; i < 3; ++i) {
         ph.dx[i] = (real)rc.dx[i];
         ph.rdx[i] = (real)1 / ph.dx[i];
+        hostDivisor(ph.dx[i], ph.dxDiv[i]);
     }
     ph.gamma = (real)rc.gamma;
     ph.cfl = rc.cfg.cfl;

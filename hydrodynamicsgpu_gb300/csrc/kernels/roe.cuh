@@ -69,11 +69,11 @@ __device__ __forceinline__ void roePrim(const real* s, real gamma, RoePrim<real,
     const int E = D + 1;
     const real gm1 = gamma - (real)1.f;
     real rho = s[0];
-    real invDensity = divI((real)1.f, rho);                              // `1.f / density`
-    // VELOCITY(ptr) = (m..., 0)/rho componentwise (res/include/HydroGPU/Euler.h:6-12);
-    // m/rho by the correction step on RN(1/rho) (fp64ops.cuh) is the same quotient
+    const Divisor<real> byRho = divisorOf(rho);
+    real invDensity = quotBy((real)1.f, byRho);                          // `1.f / density`
+    // VELOCITY(ptr) = (m..., 0)/rho componentwise (res/include/HydroGPU/Euler.h:6-12)
 #pragma unroll
-    for (int k = 0; k < D; ++k) P.v[k] = divByRecip(s[1 + k], rho, invDensity);
+    for (int k = 0; k < D; ++k) P.v[k] = quotBy(s[1 + k], byRho);
     // dot(v,v) over 4 components; the zero components add +0 to a non-negative sum
     real vv = mulN(P.v[0], P.v[0]);
 #pragma unroll

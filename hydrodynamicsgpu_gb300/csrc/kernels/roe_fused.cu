@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kThreadsX, kBlocksX)
 #pragma unroll
         for (int j = 0; j < N; ++j) {
             const double df = sF[(t + 1) * N + j] - sF[t * N + j];
-            out[j] = zfix(-divByRecip(df, ph.dx[0], ph.rdx[0]));
+            out[j] = zfix(-quotBy(df, ph.dxDiv[0]));
         }
     }
 }
