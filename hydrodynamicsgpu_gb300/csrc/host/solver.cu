@@ -500,7 +500,10 @@ void Solver<real>::initBuffers() {                           // Solver::initBuff
     healthBuf = DeviceBuffer(sizeof(unsigned), true);
     health = healthBuf.as<unsigned>();
     potential = DeviceBuffer(sizeof(real) * (size_t)rc.grid.V, true);
-    if (rc.cfg.use_gravity) relaxRhs = DeviceBuffer(sizeof(double) * (size_t)rc.grid.V, true);
+    if (rc.cfg.use_gravity) {
+        relaxRhs = DeviceBuffer(sizeof(double) * (size_t)rc.grid.V, true);
+        relaxQuot = DeviceBuffer(sizeof(real) * (size_t)rc.grid.V * relaxQuotPlanes<real>(rc.grid, gc), true);
+    }
 }
 
 // Converter::toGPU (Solver.cpp:333-337) then SelfGravitation::resetState
@@ -542,16 +545,18 @@ void Solver<real>::relaxPotential(const real* densitySource, int sweeps) {
     launch("poisson_relax_rhs", 1, [&] {
         launchRelaxRhs<real>(rc.grid, gc, densitySource, relaxRhs.template as<double>(), stream);
     });
-    auto sweep = [&] {
+    // the potential is read by the first sweep and the ghost fill, and left by the last
+    auto sweep = [&](int i) {
         launch("poisson_relax", 2, [&] {
-            launchRelaxSweep<real>(rc.grid, gc, relaxRhs.template as<double>(), potential.as<real>(), stream);
+            launchRelaxSweep<real>(rc.grid, gc, relaxRhs.template as<double>(), relaxQuot.template as<real>(),
+                                   potential.as<real>(), i == 0, i >= sweeps - 2, stream);
         });
     };
-    for (int i = 0; i < sweeps - 1; ++i) sweep();
+    for (int i = 0; i < sweeps - 1; ++i) sweep(i);
     launch("potential_boundary", rc.dim, [&] {
         launchPotentialBoundary<real>(rc.grid, methods, potential.as<real>(), stream);
     });
-    sweep();
+    sweep(sweeps - 1);
 }
 
 template <typename real>

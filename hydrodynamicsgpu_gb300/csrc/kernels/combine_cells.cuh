@@ -107,7 +107,7 @@ __device__ __forceinline__ void combinePlanCell(const real* d, const CombinePlan
 // Flux divergence and Runge-Kutta combine of one cell (res/CalcFluxDeriv.cl:7-44 and
 // the multAdd chain).  `off` is the cell offset of this grid inside the slot arrays
 // (0 for a single problem; the problem's first cell in a batch).
-// deltaFlux / dx with dx's reciprocal bits from the host (quotBy): KH 2048^2 FP64 @C1@ us
+// deltaFlux / dx with dx's reciprocal bits from the host (quotBy): KH 2048^2 FP64 237 us
 // a launch, 286 us with the x quotients by Markstein's two FMAs on the FP64 unit and the
 // rest by divI.
 template <typename real, int D, bool FLATD = false>

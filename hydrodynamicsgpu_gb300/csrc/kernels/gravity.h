@@ -27,9 +27,14 @@ void launchPotentialBoundary(const Grid& g, const int methods[3][2], real* pot, 
 // rhs = 4. * M_PI * G * density of every cell (double), from the state the sweeps relax against
 template <typename real>
 void launchRelaxRhs(const Grid& g, const GravityConst<real>& gc, const real* state, double* rhs, cudaStream_t st);
-// one gravityPotentialPoissonRelax launch in the red-black order (two kernels)
+// one gravityPotentialPoissonRelax launch in the red-black order (two kernels).  quot:
+// relaxQuotPlanes planes of V values, kept between the sweeps of one callback, the first
+// of which (`first`) reads the potential; `store`: leave the potential in `pot`.
 template <typename real>
-void launchRelaxSweep(const Grid& g, const GravityConst<real>& gc, const double* rhs, real* pot, cudaStream_t st);
+int relaxQuotPlanes(const Grid& g, const GravityConst<real>& gc);
+template <typename real>
+void launchRelaxSweep(const Grid& g, const GravityConst<real>& gc, const double* rhs, real* quot, real* pot, bool first,
+                      bool store, cudaStream_t st);
 // calcGravityDeriv of the stage state, fused with the integrator's combine
 template <typename real>
 void launchGravityCombine(const Grid& g, const GravityConst<real>& gc, const real* stage, const real* pot,
