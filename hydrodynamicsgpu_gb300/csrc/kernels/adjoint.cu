@@ -15,6 +15,7 @@
 // the branch the forward selected (dual numbers through the same min/max choices).
 // All cotangents are gathered, not scattered: every kernel writes only its own face or cell.
 #include "adjoint.h"
+#include "launch.cuh"
 #include "common.cuh"
 #include "roe.cuh"
 #include "roe_cells.cuh"
@@ -198,6 +199,7 @@ __global__ void __launch_bounds__(kT, 4) adjFluxKernel(Grid g, Phys<double> ph, 
                                                     const double* __restrict__ U, const double* __restrict__ DQ,
                                                     const double* __restrict__ B, const double* __restrict__ FT,
                                                     AdjStage st, AdjScratch S, int first) {
+    dependentLaunch();
     const int N = D + 2;
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
@@ -256,6 +258,7 @@ __device__ __forceinline__ void adjDeltaQFace(const Grid& g, double gm1, const d
 template <int D>
 __global__ void __launch_bounds__(kT) adjDeltaQKernel(Grid g, Phys<double> ph, const double* __restrict__ U,
                                                       const double* __restrict__ B, AdjScratch S) {
+    dependentLaunch();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
     int x, y, z;
@@ -270,6 +273,7 @@ __global__ void __launch_bounds__(kT) adjDeltaQKernel(Grid g, Phys<double> ph, c
 // left cell of face c + step on every axis)
 template <int D>
 __global__ void __launch_bounds__(kT) adjCellsKernel(Grid g, AdjStage st, AdjScratch S, double* __restrict__ out) {
+    dependentLaunch();
     const int N = D + 2;
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
@@ -361,6 +365,7 @@ __device__ __forceinline__ void adjBasisFace(const Grid& g, const Phys<double>& 
 template <int D>
 __global__ void __launch_bounds__(kT) adjBasisKernel(Grid g, Phys<double> ph, const double* __restrict__ U,
                                                      AdjScratch S) {
+    dependentLaunch();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
     int x, y, z;
@@ -375,6 +380,7 @@ __global__ void __launch_bounds__(kT) adjBasisKernel(Grid g, Phys<double> ph, co
 template <int D>
 __global__ void __launch_bounds__(kT) adjPrimsKernel(Grid g, Phys<double> ph, const double* __restrict__ U,
                                                      AdjScratch S, double* __restrict__ lam) {
+    dependentLaunch();
     const int N = D + 2, P = D + 2, E = N - 1;
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
@@ -427,6 +433,7 @@ __global__ void __launch_bounds__(kT) adjPrimsKernel(Grid g, Phys<double> ph, co
 
 // transposed ghost fill of one line along `axis` (boundaryLine run backwards)
 __global__ void adjBoundaryKernel(Grid g, int axis, int N, int mMin, int mMax, double* __restrict__ lam) {
+    dependentLaunch();
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int A = axis == 0 ? 1 : 0, B = axis == 2 ? 1 : 2;
     long long nA = g.S[A], nB = g.S[B];
@@ -468,7 +475,7 @@ __global__ void adjBoundaryKernel(Grid g, int axis, int N, int mMin, int mMax, d
 void launchAdjFlux(const Grid& g, const Phys<double>& ph, int limiter, const double* dtdx, const double* stage,
                    const double* dq, const double* basis, const double* fluxTape, const AdjStage& st,
                    const AdjScratch& s, int first, cudaStream_t stream) {
-#define L(DD) adjFluxKernel<DD><<<blocksFor(g.V), kT, 0, stream>>>(g, ph, limiter, dtdx[0], dtdx[1], dtdx[2], stage, dq, basis, fluxTape, st, s, first)
+#define L(DD) launchDependent(adjFluxKernel<DD>, blocksFor(g.V), kT, 0, stream, g, ph, limiter, dtdx[0], dtdx[1], dtdx[2], stage, dq, basis, fluxTape, st, s, first)
     if (g.dim == 1) { L(1); }
     else if (g.dim == 2) { L(2); }
     else { L(3); }
@@ -477,7 +484,7 @@ void launchAdjFlux(const Grid& g, const Phys<double>& ph, int limiter, const dou
 
 void launchAdjDeltaQ(const Grid& g, const Phys<double>& ph, const double* stage, const double* basis,
                      const AdjScratch& s, cudaStream_t stream) {
-#define L(DD) adjDeltaQKernel<DD><<<blocksFor(g.V), kT, 0, stream>>>(g, ph, stage, basis, s)
+#define L(DD) launchDependent(adjDeltaQKernel<DD>, blocksFor(g.V), kT, 0, stream, g, ph, stage, basis, s)
     if (g.dim == 1) L(1);
     else if (g.dim == 2) L(2);
     else L(3);
@@ -485,7 +492,7 @@ void launchAdjDeltaQ(const Grid& g, const Phys<double>& ph, const double* stage,
 }
 
 void launchAdjCells(const Grid& g, const AdjStage& st, const AdjScratch& s, double* lamOut, cudaStream_t stream) {
-#define L(DD) adjCellsKernel<DD><<<blocksFor(g.V), kT, 0, stream>>>(g, st, s, lamOut)
+#define L(DD) launchDependent(adjCellsKernel<DD>, blocksFor(g.V), kT, 0, stream, g, st, s, lamOut)
     if (g.dim == 1) L(1);
     else if (g.dim == 2) L(2);
     else L(3);
@@ -494,7 +501,7 @@ void launchAdjCells(const Grid& g, const AdjStage& st, const AdjScratch& s, doub
 
 void launchAdjBasis(const Grid& g, const Phys<double>& ph, const double* u0, const AdjScratch& s,
                     cudaStream_t stream) {
-#define L(DD) adjBasisKernel<DD><<<blocksFor(g.V), kT, 0, stream>>>(g, ph, u0, s)
+#define L(DD) launchDependent(adjBasisKernel<DD>, blocksFor(g.V), kT, 0, stream, g, ph, u0, s)
     if (g.dim == 1) L(1);
     else if (g.dim == 2) L(2);
     else L(3);
@@ -503,7 +510,7 @@ void launchAdjBasis(const Grid& g, const Phys<double>& ph, const double* u0, con
 
 void launchAdjPrims(const Grid& g, const Phys<double>& ph, const double* u0, const AdjScratch& s, double* lam,
                     cudaStream_t stream) {
-#define L(DD) adjPrimsKernel<DD><<<blocksFor(g.V), kT, 0, stream>>>(g, ph, u0, s, lam)
+#define L(DD) launchDependent(adjPrimsKernel<DD>, blocksFor(g.V), kT, 0, stream, g, ph, u0, s, lam)
     if (g.dim == 1) L(1);
     else if (g.dim == 2) L(2);
     else L(3);
@@ -514,7 +521,7 @@ void launchAdjBoundary(const Grid& g, const int methods[3][2], double* lam, cuda
     for (int axis = g.dim - 1; axis >= 0; --axis) {
         int A = axis == 0 ? 1 : 0, B = axis == 2 ? 1 : 2;
         long long lines = g.dim == 1 ? 1 : (long long)g.S[A] * g.S[B];
-        adjBoundaryKernel<<<blocksFor(lines), kT, 0, stream>>>(g, axis, g.dim + 2, methods[axis][0], methods[axis][1],
+        launchDependent(adjBoundaryKernel, blocksFor(lines), kT, 0, stream, g, axis, g.dim + 2, methods[axis][0], methods[axis][1],
                                                                lam);
     }
 }

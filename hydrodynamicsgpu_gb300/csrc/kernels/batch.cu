@@ -8,6 +8,7 @@
 // arithmetic is the single-problem code (roe_cells.cuh, hllc_cells.cuh,
 // combine_cells.cuh), so a batched problem is bit-identical to the same problem run alone.
 #include "../../../include/hgpu/hgpu.h"
+#include "launch.cuh"
 #include "batch.h"
 #include "combine_cells.cuh"
 #include "hllc_cells.cuh"
@@ -23,6 +24,7 @@ namespace {
 template <typename real, int D>
 __global__ void __launch_bounds__(256) batchBoundaryKernel(const BatchProblem<real>* __restrict__ P, int nP,
                                                            real* __restrict__ state, unsigned* q) {
+    dependentLaunch();
     for (;;) {
         int p = nextItem(q);
         if (p >= nP) break;
@@ -43,6 +45,7 @@ __global__ void __launch_bounds__(256) batchRoeBasisKernel(const BatchProblem<re
                                                            const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
                                                            int loA, int hiA, const real* __restrict__ state,
                                                            real* __restrict__ basis, unsigned* q) {
+    dependentLaunch();
     extern __shared__ unsigned char smem[];
     RoePrim<real, D>* prim = reinterpret_cast<RoePrim<real, D>*>(smem);
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
@@ -82,6 +85,7 @@ __global__ void __launch_bounds__(256) batchDtKernel(const BatchProblem<real>* _
                                                      const BatchTile* __restrict__ tiles, int nT, BatchTuning tu, int hllc,
                                                      const real* __restrict__ faces, unsigned long long* acc,
                                                      unsigned* health, unsigned* q) {
+    dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
         const BatchTile tl = tiles[t];
         const BatchProblem<real>& pr = P[tl.p];
@@ -104,6 +108,7 @@ __global__ void __launch_bounds__(256) batchDtKernel(const BatchProblem<real>* _
 template <typename real>
 __global__ void batchFinalizeKernel(const BatchProblem<real>* __restrict__ P, int nP, int integ,
                                     unsigned long long* acc, StepConst<real>* sc) {
+    dependentLaunch();
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= nP) return;
     const BatchProblem<real>& pr = P[p];
@@ -116,6 +121,7 @@ __global__ void __launch_bounds__(256) batchDeltaQKernel(const BatchProblem<real
                                                          int loA, int hiA, const real* __restrict__ stage,
                                                          const real* __restrict__ basis, real* __restrict__ dq,
                                                          unsigned* q) {
+    dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
         const BatchTile tl = tiles[t];
         const BatchProblem<real>& pr = P[tl.p];
@@ -135,6 +141,7 @@ __global__ void __launch_bounds__(256, PLAIN ? 5 : 1) batchCombineKernel(const B
                                                           const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
                                                           const real* __restrict__ flux, CombinePlan<real> plan,
                                                           const StepConst<real>* __restrict__ sc, unsigned* q) {
+    dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
         const BatchTile tl = tiles[t];
         const BatchProblem<real>& pr = P[tl.p];
@@ -154,6 +161,7 @@ __global__ void __launch_bounds__(256) batchGravityKernel(const BatchProblem<rea
                                                           const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
                                                           int integ, const StepConst<real>* __restrict__ sc,
                                                           real* __restrict__ state, unsigned* q) {
+    dependentLaunch();
     for (int t = firstItem(q, tu); t < nT; t = nextItemAfter(q, tu)) {
         const BatchTile tl = tiles[t];
         const BatchProblem<real>& pr = P[tl.p];
@@ -177,6 +185,7 @@ __global__ void __launch_bounds__(256) batchStateCheckKernel(const BatchProblem<
                                                              const BatchTile* __restrict__ tiles, int nT,
                                                              BatchTuning tu, const real* __restrict__ state,
                                                              unsigned* health, unsigned* healthP, unsigned* q) {
+    dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
         const BatchTile tl = tiles[t];
         const BatchProblem<real>& pr = P[tl.p];
@@ -196,6 +205,7 @@ __global__ void __launch_bounds__(256) batchWaveKernel(const BatchProblem<real>*
                                                        const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
                                                        const real* __restrict__ state, real* __restrict__ waves,
                                                        unsigned* q) {
+    dependentLaunch();
     for (int t = firstItem(q, tu); t < nT; t = nextItemAfter(q, tu)) {
         const BatchTile tl = tiles[t];
         const BatchProblem<real>& pr = P[tl.p];
@@ -214,9 +224,9 @@ __global__ void __launch_bounds__(256) batchWaveKernel(const BatchProblem<real>*
 
 template <typename real>
 void BatchLaunch<real>::boundary(unsigned* q) const {
-    if (dim == 1) batchBoundaryKernel<real, 1><<<persistentBlocks(batchBoundaryKernel<real, 1>, 0, tu.blocksPerSM, nP), 256, 0, st>>>(P, nP, state, q);
-    else if (dim == 2) batchBoundaryKernel<real, 2><<<persistentBlocks(batchBoundaryKernel<real, 2>, 0, tu.blocksPerSM, nP), 256, 0, st>>>(P, nP, state, q);
-    else batchBoundaryKernel<real, 3><<<persistentBlocks(batchBoundaryKernel<real, 3>, 0, tu.blocksPerSM, nP), 256, 0, st>>>(P, nP, state, q);
+    if (dim == 1) launchDependent(batchBoundaryKernel<real, 1>, persistentBlocks(batchBoundaryKernel<real, 1>, 0, tu.blocksPerSM, nP), 256, 0, st, P, nP, state, q);
+    else if (dim == 2) launchDependent(batchBoundaryKernel<real, 2>, persistentBlocks(batchBoundaryKernel<real, 2>, 0, tu.blocksPerSM, nP), 256, 0, st, P, nP, state, q);
+    else launchDependent(batchBoundaryKernel<real, 3>, persistentBlocks(batchBoundaryKernel<real, 3>, 0, tu.blocksPerSM, nP), 256, 0, st, P, nP, state, q);
 }
 
 template <typename real>
@@ -231,10 +241,9 @@ void BatchLaunch<real>::roeBasis(int loA, int hiA, unsigned* q) const {
     int smem = tu.staged ? primSmem<real>(dim, tu) : 0;
 #define L(DD)                                                                                                      \
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                                        \
-        batchRoeBasisKernel<real, DD, true><<<nT, 256, smem, st>>>(P, tiles, nT, tu, loA, hiA, state, faces, q);    \
+        launchDependent(batchRoeBasisKernel<real, DD, true>, nT, 256, smem, st, P, tiles, nT, tu, loA, hiA, state, faces, q);    \
     else                                                                                                           \
-        batchRoeBasisKernel<real, DD, false><<<persistentBlocks(batchRoeBasisKernel<real, DD, false>, smem,         \
-                                                                tu.blocksPerSM, nT), 256, smem, st>>>(              \
+        launchDependent(batchRoeBasisKernel<real, DD, false>, persistentBlocks(batchRoeBasisKernel<real, DD, false>, smem, tu.blocksPerSM, nT), 256, smem, st,               \
             P, tiles, nT, tu, loA, hiA, state, faces, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }
@@ -244,7 +253,7 @@ void BatchLaunch<real>::roeBasis(int loA, int hiA, unsigned* q) const {
 
 template <typename real>
 void BatchLaunch<real>::waves(int hll, unsigned* q) const {
-#define L(DD, H) batchWaveKernel<real, DD, H><<<persistentBlocks(batchWaveKernel<real, DD, H>, 0, tu.blocksPerSM, nT), 256, 0, st>>>(P, tiles, nT, tu, state, faces, q)
+#define L(DD, H) launchDependent(batchWaveKernel<real, DD, H>, persistentBlocks(batchWaveKernel<real, DD, H>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, state, faces, q)
     if (hll) {
         if (dim == 1) L(1, true);
         else if (dim == 2) L(2, true);
@@ -261,10 +270,9 @@ template <typename real>
 void BatchLaunch<real>::dt(int hllc, unsigned long long* acc, unsigned* health, unsigned* q) const {
 #define L(DD)                                                                                                      \
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                         \
-        batchDtKernel<real, DD, true><<<nT, 256, 0, st>>>(P, tiles, nT, tu, hllc, faces, acc, health, q);           \
+        launchDependent(batchDtKernel<real, DD, true>, nT, 256, 0, st, P, tiles, nT, tu, hllc, faces, acc, health, q);           \
     else                                                                                                           \
-        batchDtKernel<real, DD, false><<<persistentBlocks(batchDtKernel<real, DD, false>, 0, tu.blocksPerSM, nT),   \
-                                         256, 0, st>>>(P, tiles, nT, tu, hllc, faces, acc, health, q)
+        launchDependent(batchDtKernel<real, DD, false>, persistentBlocks(batchDtKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, hllc, faces, acc, health, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }
     else { L(3); }
@@ -273,17 +281,16 @@ void BatchLaunch<real>::dt(int hllc, unsigned long long* acc, unsigned* health, 
 
 template <typename real>
 void BatchLaunch<real>::finalize(int integ, unsigned long long* acc, StepConst<real>* sc) const {
-    batchFinalizeKernel<real><<<(nP + 127) / 128, 128, 0, st>>>(P, nP, integ, acc, sc);
+    launchDependent(batchFinalizeKernel<real>, (nP + 127) / 128, 128, 0, st, P, nP, integ, acc, sc);
 }
 
 template <typename real>
 void BatchLaunch<real>::deltaQ(int loA, int hiA, const real* stage, real* dq, unsigned* q) const {
 #define L(DD)                                                                                                      \
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                                        \
-        batchDeltaQKernel<real, DD, true><<<nT, 256, 0, st>>>(P, tiles, nT, tu, loA, hiA, stage, faces, dq, q);     \
+        launchDependent(batchDeltaQKernel<real, DD, true>, nT, 256, 0, st, P, tiles, nT, tu, loA, hiA, stage, faces, dq, q);     \
     else                                                                                                           \
-        batchDeltaQKernel<real, DD, false><<<persistentBlocks(batchDeltaQKernel<real, DD, false>, 0, tu.blocksPerSM, \
-                                                              nT), 256, 0, st>>>(P, tiles, nT, tu, loA, hiA, stage,  \
+        launchDependent(batchDeltaQKernel<real, DD, false>, persistentBlocks(batchDeltaQKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, loA, hiA, stage,  \
                                                                                  faces, dq, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }
@@ -296,10 +303,9 @@ void BatchLaunch<real>::combine(const real* fluxBuf, const CombinePlan<real>& pl
                                 unsigned* q) const {
 #define L(DD)                                                                                                      \
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                                        \
-        batchCombineKernel<real, DD, true><<<nT, 256, 0, st>>>(P, tiles, nT, tu, fluxBuf, plan, sc, q);             \
+        launchDependent(batchCombineKernel<real, DD, true>, nT, 256, 0, st, P, tiles, nT, tu, fluxBuf, plan, sc, q);             \
     else                                                                                                           \
-        batchCombineKernel<real, DD, false><<<persistentBlocks(batchCombineKernel<real, DD, false>, 0,              \
-                                                               tu.blocksPerSM, nT), 256, 0, st>>>(P, tiles, nT, tu,  \
+        launchDependent(batchCombineKernel<real, DD, false>, persistentBlocks(batchCombineKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu,  \
                                                                                                   fluxBuf, plan, sc, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }
@@ -309,7 +315,7 @@ void BatchLaunch<real>::combine(const real* fluxBuf, const CombinePlan<real>& pl
 
 template <typename real>
 void BatchLaunch<real>::gravity(int integ, const StepConst<real>* sc, unsigned* q) const {
-#define L(DD) batchGravityKernel<real, DD><<<persistentBlocks(batchGravityKernel<real, DD>, 0, tu.blocksPerSM, nT), 256, 0, st>>>(P, tiles, nT, tu, integ, sc, state, q)
+#define L(DD) launchDependent(batchGravityKernel<real, DD>, persistentBlocks(batchGravityKernel<real, DD>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, integ, sc, state, q)
     if (dim == 1) L(1);
     else if (dim == 2) L(2);
     else L(3);
@@ -320,10 +326,9 @@ template <typename real>
 void BatchLaunch<real>::stateCheck(unsigned* health, unsigned* healthP, unsigned* q) const {
 #define L(DD)                                                                                                      \
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                         \
-        batchStateCheckKernel<real, DD, true><<<nT, 256, 0, st>>>(P, tiles, nT, tu, state, health, healthP, q);     \
+        launchDependent(batchStateCheckKernel<real, DD, true>, nT, 256, 0, st, P, tiles, nT, tu, state, health, healthP, q);     \
     else                                                                                                           \
-        batchStateCheckKernel<real, DD, false><<<persistentBlocks(batchStateCheckKernel<real, DD, false>, 0,        \
-                                                                  tu.blocksPerSM, nT), 256, 0, st>>>(               \
+        launchDependent(batchStateCheckKernel<real, DD, false>, persistentBlocks(batchStateCheckKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st,                \
             P, tiles, nT, tu, state, health, healthP, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }

@@ -1,6 +1,7 @@
 // batch_flux.cu -- the batched interface-flux kernels (one translation unit of their
 // own: they are instantiated per solver and slope limiter).  See batch.cu.
 #include "../../../include/hgpu/hgpu.h"
+#include "launch.cuh"
 #include "batch.h"
 #include "batch_common.cuh"
 #include "hllc_cells.cuh"
@@ -19,6 +20,7 @@ __global__ void __launch_bounds__(256) batchFluxKernel(const BatchProblem<real>*
                                                        const real* __restrict__ stage, const real* __restrict__ faces,
                                                        const real* __restrict__ dq, real* __restrict__ flux,
                                                        unsigned* health, unsigned* q) {
+    dependentLaunch();
     for (int t = firstItem(q, tu); t < nT; t = nextItemAfter(q, tu)) {
         const BatchTile tl = tiles[t];
         const BatchProblem<real>& pr = P[tl.p];
@@ -51,6 +53,7 @@ __global__ void __launch_bounds__(256) batchFluxCorrKernel(const BatchProblem<do
                                                            const double* __restrict__ faces,
                                                            const double* __restrict__ dq, double* __restrict__ flux,
                                                            unsigned* q) {
+    dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
         const BatchTile tl = tiles[t];
         const BatchProblem<double>& pr = P[tl.p];
@@ -72,6 +75,7 @@ __global__ void __launch_bounds__(256, PLAIN && D <= 2 ? 3 : 1) batchFluxXformKe
                                                             const double* __restrict__ stage,
                                                             const double* __restrict__ faces,
                                                             double* __restrict__ flux, unsigned* q) {
+    dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
         const BatchTile tl = tiles[t];
         const BatchProblem<double>& pr = P[tl.p];
@@ -92,8 +96,7 @@ template <typename real, int HLLC, int LIM>
 static void batchFluxLaunch(const BatchLaunch<real>& b, int hllc, int lim, const StepConst<real>* sc,
                             const real* stage, const real* dq, real* fluxBuf, unsigned* health, unsigned* q) {
 #define L(DD)                                                                                                       \
-    batchFluxKernel<real, DD, HLLC, LIM><<<persistentBlocks(batchFluxKernel<real, DD, HLLC, LIM>, 0, b.tu.blocksPerSM, b.nT), \
-                                           256, 0, b.st>>>(b.P, b.tiles, b.nT, b.tu, hllc, lim, sc, stage, b.faces, dq, \
+    launchDependent(batchFluxKernel<real, DD, HLLC, LIM>, persistentBlocks(batchFluxKernel<real, DD, HLLC, LIM>, 0, b.tu.blocksPerSM, b.nT), 256, 0, b.st, b.P, b.tiles, b.nT, b.tu, hllc, lim, sc, stage, b.faces, dq, \
                                                            fluxBuf, health, q)
     if (b.dim == 1) L(1);
     else if (b.dim == 2) L(2);
@@ -121,14 +124,12 @@ static void batchFluxSplitLaunch(const BatchProblem<double>* P, const BatchTile*
                                  const double* stage, const double* dq, double* fluxBuf, unsigned* q0, unsigned* q1) {
 #define L(DD)                                                                                                       \
     if (tu.blocksPerSM < 0 && tu.cpt == 1) {                                                                                       \
-        batchFluxCorrKernel<DD, LIM, true><<<nT, 256, 0, st>>>(P, tiles, nT, tu, lim, sc, faces, dq, fluxBuf, q0);   \
-        batchFluxXformKernel<DD, true><<<nT, 256, 0, st>>>(P, tiles, nT, tu, stage, faces, fluxBuf, q1);             \
+        launchDependent(batchFluxCorrKernel<DD, LIM, true>, nT, 256, 0, st, P, tiles, nT, tu, lim, sc, faces, dq, fluxBuf, q0);   \
+        launchDependent(batchFluxXformKernel<DD, true>, nT, 256, 0, st, P, tiles, nT, tu, stage, faces, fluxBuf, q1);             \
     } else {                                                                                                        \
-        batchFluxCorrKernel<DD, LIM, false><<<persistentBlocks(batchFluxCorrKernel<DD, LIM, false>, 0,               \
-                                                               tu.blocksPerSM, nT), 256, 0, st>>>(                  \
+        launchDependent(batchFluxCorrKernel<DD, LIM, false>, persistentBlocks(batchFluxCorrKernel<DD, LIM, false>, 0, tu.blocksPerSM, nT), 256, 0, st,                   \
             P, tiles, nT, tu, lim, sc, faces, dq, fluxBuf, q0);                                                     \
-        batchFluxXformKernel<DD, false><<<persistentBlocks(batchFluxXformKernel<DD, false>, 0, tu.blocksPerSM, nT),  \
-                                          256, 0, st>>>(P, tiles, nT, tu, stage, faces, fluxBuf, q1);               \
+        launchDependent(batchFluxXformKernel<DD, false>, persistentBlocks(batchFluxXformKernel<DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, stage, faces, fluxBuf, q1);               \
     }
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }

@@ -13,6 +13,7 @@
 //    finalised on the device, with dt/dx and beta*dt, for the whole step.
 #include "combine_cells.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace hgpu {
 
@@ -35,6 +36,7 @@ inline unsigned blocksFor(long long n) { return (unsigned)((n + kThreads - 1) / 
 template <typename real>
 __global__ void __launch_bounds__(kThreads) boundaryKernel(Grid g, int axis, int N, int mMin, int mMax,
                                                            real* __restrict__ state, long long t0, long long t1) {
+    dependentLaunch();
     const long long t = t0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= t1) return;
     boundaryLine<real>(g, axis, N, mMin, mMax, state, t);
@@ -47,6 +49,7 @@ __global__ void __launch_bounds__(kThreads, 5) derivCombineKernel(Grid g, Phys<r
                                                                CombinePlan<real> plan,
                                                                const StepConst<real>* __restrict__ sc, long long c0,
                                                                long long c1) {
+    dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
     int x, y, z;
@@ -57,6 +60,7 @@ __global__ void __launch_bounds__(kThreads, 5) derivCombineKernel(Grid g, Phys<r
 template <typename real>
 __global__ void __launch_bounds__(kThreads) alphaOnlyKernel(long long n, int integ, real* __restrict__ state,
                                                             const StepConst<real>* __restrict__ sc) {
+    dependentLaunch();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     state[i] = alphaOnlyElem<real>(integ, state[i], *sc);
@@ -65,17 +69,19 @@ __global__ void __launch_bounds__(kThreads) alphaOnlyKernel(long long n, int int
 template <typename real>
 __global__ void finalizeDtKernel(Phys<real> ph, int integ, int useFixed, double fixedDt, unsigned long long* acc,
                                  unsigned long long accInit, StepConst<real>* sc) {
+    dependentLaunch();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     finalizeOne<real>(ph, integ, useFixed, fixedDt, acc, accInit, sc);
 }
 
-__global__ void resetAccKernel(unsigned long long* acc, unsigned long long v) { *acc = v; }
+__global__ void resetAccKernel(unsigned long long* acc, unsigned long long v) { dependentLaunch(); *acc = v; }
 
 // Self-gravity pass with ForwardEuler and a zero potential: the (ghost-refreshed)
 // state gets `state + deriv * dt` with deriv == +0 (ForwardEuler.cpp:20-32).
 template <typename real>
 __global__ void __launch_bounds__(kThreads) zeroAddKernel(long long n, real* __restrict__ state,
                                                           const StepConst<real>* __restrict__ sc) {
+    dependentLaunch();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     state[i] = state[i] + (real)0. * sc->dt;
@@ -94,7 +100,7 @@ void launchBoundaryAxis(const Grid& g, const int methods[3][2], real* state, cud
     if (t1 < 0 || t1 > n) t1 = n;
     if (t0 < 0) t0 = 0;
     if (t0 >= t1) return;
-    boundaryKernel<real><<<blocksFor(t1 - t0), kThreads, 0, st>>>(g, axis, g.dim + 2, methods[axis][0],
+    launchDependent(boundaryKernel<real>, blocksFor(t1 - t0), kThreads, 0, st, g, axis, g.dim + 2, methods[axis][0],
                                                                    methods[axis][1], state, t0, t1);
 }
 
@@ -110,33 +116,33 @@ void launchDerivCombine(const Grid& g, const Phys<real>& ph, const real* flux, c
     if (c0 < 0) c0 = 0;
     if (c0 >= c1) return;
     const unsigned b = blocksFor(c1 - c0);
-    if (g.dim == 1) derivCombineKernel<real, 1><<<b, kThreads, 0, st>>>(g, ph, flux, plan, sc, c0, c1);
-    else if (g.dim == 2) derivCombineKernel<real, 2><<<b, kThreads, 0, st>>>(g, ph, flux, plan, sc, c0, c1);
-    else derivCombineKernel<real, 3><<<b, kThreads, 0, st>>>(g, ph, flux, plan, sc, c0, c1);
+    if (g.dim == 1) launchDependent(derivCombineKernel<real, 1>, b, kThreads, 0, st, g, ph, flux, plan, sc, c0, c1);
+    else if (g.dim == 2) launchDependent(derivCombineKernel<real, 2>, b, kThreads, 0, st, g, ph, flux, plan, sc, c0, c1);
+    else launchDependent(derivCombineKernel<real, 3>, b, kThreads, 0, st, g, ph, flux, plan, sc, c0, c1);
 }
 
 template <typename real>
 void launchAlphaOnly(const Grid& g, int integrator, real* state, const StepConst<real>* sc, cudaStream_t st) {
     long long n = g.V * (g.dim + 2);
-    alphaOnlyKernel<real><<<blocksFor(n), kThreads, 0, st>>>(n, integrator, state, sc);
+    launchDependent(alphaOnlyKernel<real>, blocksFor(n), kThreads, 0, st, n, integrator, state, sc);
 }
 
 template <typename real>
 void launchZeroAdd(const Grid& g, real* state, const StepConst<real>* sc, cudaStream_t st) {
     long long n = g.V * (g.dim + 2);
-    zeroAddKernel<real><<<blocksFor(n), kThreads, 0, st>>>(n, state, sc);
+    launchDependent(zeroAddKernel<real>, blocksFor(n), kThreads, 0, st, n, state, sc);
 }
 
 template <typename real>
 void launchFinalizeDt(const Phys<real>& ph, int integrator, int useFixed, double fixedDt, unsigned long long* acc,
                       unsigned long long accInit, StepConst<real>* sc, unsigned* health, cudaStream_t st) {
     (void)health;
-    finalizeDtKernel<real><<<1, 32, 0, st>>>(ph, integrator, useFixed, fixedDt, acc, accInit, sc);
+    launchDependent(finalizeDtKernel<real>, 1, 32, 0, st, ph, integrator, useFixed, fixedDt, acc, accInit, sc);
 }
 
 template <typename real>
 void launchResetAcc(unsigned long long* acc, unsigned long long accInit, cudaStream_t st) {
-    resetAccKernel<<<1, 1, 0, st>>>(acc, accInit);
+    launchDependent(resetAccKernel, 1, 1, 0, st, acc, accInit);
 }
 
 #define INST(real)                                                                                              \

@@ -22,6 +22,7 @@
 // double literals of `4. * M_PI * G * density`, `-2. * (1. / (DX * DX) ...)` and
 // `/ (2. * dx[side])` promote those expressions to double.
 #include "../../../include/hgpu/hgpu.h"
+#include "launch.cuh"
 #include "combine_cells.cuh"
 #include "gravity.h"
 
@@ -35,6 +36,7 @@ inline unsigned blocksFor(long long n) { return (unsigned)((n + kThreads - 1) / 
 template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) potentialInitKernel(Grid g, int fromDensity, real* __restrict__ state,
                                                                 real* __restrict__ pot, long long c0, long long c1) {
+    dependentLaunch();
     const long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
     real* s = state + (long long)(D + 2) * c;
@@ -47,6 +49,7 @@ __global__ void __launch_bounds__(kThreads) potentialInitKernel(Grid g, int from
 template <typename real>
 __global__ void __launch_bounds__(kThreads) potentialBoundaryKernel(Grid g, int axis, int mMin, int mMax,
                                                                     real* __restrict__ pot) {
+    dependentLaunch();
     boundaryLine<real>(g, axis, 1, mMin, mMax, pot, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -56,6 +59,7 @@ __global__ void __launch_bounds__(kThreads) potentialBoundaryKernel(Grid g, int 
 template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) relaxRhsKernel(Grid g, GravityConst<real> gc,
                                                            const real* __restrict__ state, double* __restrict__ rhs) {
+    dependentLaunch();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
     rhs[c] = mulI(gc.fourPiG, (double)state[(long long)(D + 2) * c]);
@@ -76,6 +80,7 @@ template <typename real, int D, bool SAME, bool FIRST>
 __global__ void __launch_bounds__(kThreads) relaxKernel(Grid g, GravityConst<real> gc, int colour, bool store,
                                                         const double* __restrict__ rhs, real* __restrict__ quot,
                                                         real* __restrict__ pot) {
+    dependentLaunch();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = D > 1 ? (int)blockIdx.y + 2 : 0, z = D > 2 ? (int)blockIdx.z + 2 : 0;
     // x = 2 + 2k + shift, with shift chosen so that x + y + z has the colour's parity
@@ -110,6 +115,7 @@ __global__ void __launch_bounds__(kThreads) gravityCombineKernel(Grid g, Gravity
                                                                  const real* __restrict__ stage,
                                                                  const real* __restrict__ pot, CombinePlan<real> plan,
                                                                  const StepConst<real>* __restrict__ sc) {
+    dependentLaunch();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
     int x, y, z;
@@ -166,9 +172,9 @@ void launchPotentialInit(const Grid& g, int fromDensity, real* state, real* pot,
     if (c0 < 0) c0 = 0;
     if (c0 >= c1) return;
     const unsigned b = blocksFor(c1 - c0);
-    if (g.dim == 1) potentialInitKernel<real, 1><<<b, kThreads, 0, st>>>(g, fromDensity, state, pot, c0, c1);
-    else if (g.dim == 2) potentialInitKernel<real, 2><<<b, kThreads, 0, st>>>(g, fromDensity, state, pot, c0, c1);
-    else potentialInitKernel<real, 3><<<b, kThreads, 0, st>>>(g, fromDensity, state, pot, c0, c1);
+    if (g.dim == 1) launchDependent(potentialInitKernel<real, 1>, b, kThreads, 0, st, g, fromDensity, state, pot, c0, c1);
+    else if (g.dim == 2) launchDependent(potentialInitKernel<real, 2>, b, kThreads, 0, st, g, fromDensity, state, pot, c0, c1);
+    else launchDependent(potentialInitKernel<real, 3>, b, kThreads, 0, st, g, fromDensity, state, pot, c0, c1);
 }
 
 template <typename real>
@@ -178,15 +184,15 @@ void launchPotentialBoundary(const Grid& g, const int methods[3][2], real* pot, 
         for (int k = 0; k < 2; ++k)
             m[k] = methods[axis][k] == HGPU_BOUNDARY_MIRROR ? HGPU_BOUNDARY_FREEFLOW : methods[axis][k];
         const long long n = g.dim == 1 ? 1 : (long long)g.S[axis == 0 ? 1 : 0] * g.S[axis == 2 ? 1 : 2];
-        potentialBoundaryKernel<real><<<blocksFor(n), kThreads, 0, st>>>(g, axis, m[0], m[1], pot);
+        launchDependent(potentialBoundaryKernel<real>, blocksFor(n), kThreads, 0, st, g, axis, m[0], m[1], pot);
     }
 }
 
 template <typename real>
 void launchRelaxRhs(const Grid& g, const GravityConst<real>& gc, const real* state, double* rhs, cudaStream_t st) {
-    if (g.dim == 1) relaxRhsKernel<real, 1><<<blocksFor(g.V), kThreads, 0, st>>>(g, gc, state, rhs);
-    else if (g.dim == 2) relaxRhsKernel<real, 2><<<blocksFor(g.V), kThreads, 0, st>>>(g, gc, state, rhs);
-    else relaxRhsKernel<real, 3><<<blocksFor(g.V), kThreads, 0, st>>>(g, gc, state, rhs);
+    if (g.dim == 1) launchDependent(relaxRhsKernel<real, 1>, blocksFor(g.V), kThreads, 0, st, g, gc, state, rhs);
+    else if (g.dim == 2) launchDependent(relaxRhsKernel<real, 2>, blocksFor(g.V), kThreads, 0, st, g, gc, state, rhs);
+    else launchDependent(relaxRhsKernel<real, 3>, blocksFor(g.V), kThreads, 0, st, g, gc, state, rhs);
 }
 
 template <typename real, int D, bool SAME>
@@ -195,9 +201,9 @@ static void relaxSweep(const Grid& g, const GravityConst<real>& gc, const double
     const int nx = g.S[0] - 4, ny = D > 1 ? g.S[1] - 4 : 1, nz = D > 2 ? g.S[2] - 4 : 1;
     if (nx <= 0 || ny <= 0 || nz <= 0) return;
     const dim3 grid((unsigned)((nx + 1) / 2 + kThreads - 1) / kThreads, (unsigned)ny, (unsigned)nz);
-    if (first) relaxKernel<real, D, SAME, true><<<grid, kThreads, 0, st>>>(g, gc, 0, store, rhs, quot, pot);
-    else relaxKernel<real, D, SAME, false><<<grid, kThreads, 0, st>>>(g, gc, 0, store, rhs, quot, pot);
-    relaxKernel<real, D, SAME, false><<<grid, kThreads, 0, st>>>(g, gc, 1, store, rhs, quot, pot);
+    if (first) launchDependent(relaxKernel<real, D, SAME, true>, grid, kThreads, 0, st, g, gc, 0, store, rhs, quot, pot);
+    else launchDependent(relaxKernel<real, D, SAME, false>, grid, kThreads, 0, st, g, gc, 0, store, rhs, quot, pot);
+    launchDependent(relaxKernel<real, D, SAME, false>, grid, kThreads, 0, st, g, gc, 1, store, rhs, quot, pot);
 }
 
 template <typename real>
@@ -221,9 +227,9 @@ void launchRelaxSweep(const Grid& g, const GravityConst<real>& gc, const double*
 template <typename real>
 void launchGravityCombine(const Grid& g, const GravityConst<real>& gc, const real* stage, const real* pot,
                           const CombinePlan<real>& plan, const StepConst<real>* sc, cudaStream_t st) {
-    if (g.dim == 1) gravityCombineKernel<real, 1><<<blocksFor(g.V), kThreads, 0, st>>>(g, gc, stage, pot, plan, sc);
-    else if (g.dim == 2) gravityCombineKernel<real, 2><<<blocksFor(g.V), kThreads, 0, st>>>(g, gc, stage, pot, plan, sc);
-    else gravityCombineKernel<real, 3><<<blocksFor(g.V), kThreads, 0, st>>>(g, gc, stage, pot, plan, sc);
+    if (g.dim == 1) launchDependent(gravityCombineKernel<real, 1>, blocksFor(g.V), kThreads, 0, st, g, gc, stage, pot, plan, sc);
+    else if (g.dim == 2) launchDependent(gravityCombineKernel<real, 2>, blocksFor(g.V), kThreads, 0, st, g, gc, stage, pot, plan, sc);
+    else launchDependent(gravityCombineKernel<real, 3>, blocksFor(g.V), kThreads, 0, st, g, gc, stage, pot, plan, sc);
 }
 
 #define INST(real)                                                                                              \

@@ -1,6 +1,7 @@
 // health.cu -- the state check of one problem (health.cuh): after every step and
 // after every upload, over the interior cells, into the solver's health word.
 #include "health.cuh"
+#include "launch.cuh"
 
 namespace hgpu {
 
@@ -11,6 +12,7 @@ constexpr int kThreads = 256;
 template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) stateCheckKernel(Grid g, const real* __restrict__ state,
                                                              const real* __restrict__ pot, unsigned* health) {
+    dependentLaunch();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned bits = 0;
     if (c < g.V) {
@@ -26,9 +28,9 @@ __global__ void __launch_bounds__(kThreads) stateCheckKernel(Grid g, const real*
 template <typename real>
 void launchStateCheck(const Grid& g, const real* state, const real* pot, unsigned* health, cudaStream_t st) {
     const unsigned b = (unsigned)((g.V + kThreads - 1) / kThreads);
-    if (g.dim == 1) stateCheckKernel<real, 1><<<b, kThreads, 0, st>>>(g, state, pot, health);
-    else if (g.dim == 2) stateCheckKernel<real, 2><<<b, kThreads, 0, st>>>(g, state, pot, health);
-    else stateCheckKernel<real, 3><<<b, kThreads, 0, st>>>(g, state, pot, health);
+    if (g.dim == 1) launchDependent(stateCheckKernel<real, 1>, b, kThreads, 0, st, g, state, pot, health);
+    else if (g.dim == 2) launchDependent(stateCheckKernel<real, 2>, b, kThreads, 0, st, g, state, pot, health);
+    else launchDependent(stateCheckKernel<real, 3>, b, kThreads, 0, st, g, state, pot, health);
 }
 
 template void launchStateCheck<double>(const Grid&, const double*, const double*, unsigned*, cudaStream_t);

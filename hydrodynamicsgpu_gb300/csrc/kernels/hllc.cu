@@ -12,6 +12,7 @@
 // speeds and the two-state HLL flux; its timestep kernel is HLLC's.
 #include "hllc_cells.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "reduce.cuh"
 
 namespace hgpu {
@@ -24,6 +25,7 @@ template <typename real, int D, bool HLL, bool GRAV>
 __global__ void __launch_bounds__(kThreads) hllcWaveKernel(Grid g, Phys<real> ph, double gq,
                                                            const real* __restrict__ state, real* __restrict__ waves,
                                                            const real* __restrict__ pot, long long c0, long long c1) {
+    dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
     int x, y, z;
@@ -34,6 +36,7 @@ __global__ void __launch_bounds__(kThreads) hllcWaveKernel(Grid g, Phys<real> ph
 template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) hllcDtKernel(Grid g, Phys<real> ph, const real* __restrict__ waves,
                                                          unsigned long long* acc, unsigned* health) {
+    dependentLaunch();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long best = ~0ULL;
     bool nan = false;
@@ -51,6 +54,7 @@ __global__ void __launch_bounds__(kThreads) hllcFluxKernel(Grid g, Phys<real> ph
                                                            const real* __restrict__ waves, real* __restrict__ flux,
                                                            unsigned* health, const real* __restrict__ pot,
                                                            long long c0, long long c1) {
+    dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
     int x, y, z;
@@ -70,6 +74,7 @@ __global__ void __launch_bounds__(kThreads) hllcFluxTileKernel(Grid g, Phys<real
                                                                const real* __restrict__ waves,
                                                                real* __restrict__ flux, unsigned* health,
                                                                const real* __restrict__ pot, int s0, int s1) {
+    dependentLaunch();
     typedef FluxTile<D> T;
     constexpr int HX = T::X + 1, HY = T::Y + 1, HZ = D > 2 ? T::Z + 1 : 1;
     __shared__ Prim<real, D> prim[HX * HY * HZ];
@@ -91,6 +96,7 @@ __global__ void __launch_bounds__(kThreads, 1) hllcFluxTileKernelWide(Grid g, Ph
                                                                       const real* __restrict__ waves,
                                                                       real* __restrict__ flux, unsigned* health,
                                                                       const real* __restrict__ pot, int s0, int s1) {
+    dependentLaunch();
     typedef FluxTile<2> T;
     constexpr int HX = T::X + 1, HY = T::Y + 1;
     __shared__ Prim<real, 2> prim[HX * HY];
@@ -105,6 +111,7 @@ __global__ void __launch_bounds__(kThreads) hllcWaveTileKernel(Grid g, Phys<real
                                                                const real* __restrict__ state,
                                                                real* __restrict__ waves, const real* __restrict__ pot,
                                                                int s0, int s1) {
+    dependentLaunch();
     typedef FluxTile<D> T;
     constexpr int HX = T::X + 1, HY = T::Y + 1, HZ = D > 2 ? T::Z + 1 : 1;
     __shared__ Prim<real, D> prim[HX * HY * HZ];
@@ -139,7 +146,7 @@ void launchHllcWavesG(const Grid& g, const Phys<real>& ph, const real* state, re
     if (g.dim > 1 && c0 % plane == 0 && c1 % plane == 0) {
         const int s0 = (int)(c0 / plane), s1 = (int)(c1 / plane);
 #define T(DD, H) \
-    hllcWaveTileKernel<real, DD, H, GRAV><<<tileGrid<DD>(g, s0, s1), kThreads, 0, st>>>(g, ph, gq, state, waves, pot, s0, s1)
+    launchDependent(hllcWaveTileKernel<real, DD, H, GRAV>, tileGrid<DD>(g, s0, s1), kThreads, 0, st, g, ph, gq, state, waves, pot, s0, s1)
         if (hll) {
             if (g.dim == 2) T(2, true);
             else T(3, true);
@@ -151,7 +158,7 @@ void launchHllcWavesG(const Grid& g, const Phys<real>& ph, const real* state, re
         return;
     }
 #define L(DD, H) \
-    hllcWaveKernel<real, DD, H, GRAV><<<blocksFor(c1 - c0), kThreads, 0, st>>>(g, ph, gq, state, waves, pot, c0, c1)
+    launchDependent(hllcWaveKernel<real, DD, H, GRAV>, blocksFor(c1 - c0), kThreads, 0, st, g, ph, gq, state, waves, pot, c0, c1)
     if (hll) {
         if (g.dim == 1) L(1, true);
         else if (g.dim == 2) L(2, true);
@@ -174,9 +181,9 @@ void launchHllcWaves(const Grid& g, const Phys<real>& ph, const real* state, rea
 template <typename real>
 void launchHllcDt(const Grid& g, const Phys<real>& ph, const real* waves, unsigned long long* acc, unsigned* health,
                   cudaStream_t st) {
-    if (g.dim == 1) hllcDtKernel<real, 1><<<blocksFor(g.V), kThreads, 0, st>>>(g, ph, waves, acc, health);
-    else if (g.dim == 2) hllcDtKernel<real, 2><<<blocksFor(g.V), kThreads, 0, st>>>(g, ph, waves, acc, health);
-    else hllcDtKernel<real, 3><<<blocksFor(g.V), kThreads, 0, st>>>(g, ph, waves, acc, health);
+    if (g.dim == 1) launchDependent(hllcDtKernel<real, 1>, blocksFor(g.V), kThreads, 0, st, g, ph, waves, acc, health);
+    else if (g.dim == 2) launchDependent(hllcDtKernel<real, 2>, blocksFor(g.V), kThreads, 0, st, g, ph, waves, acc, health);
+    else launchDependent(hllcDtKernel<real, 3>, blocksFor(g.V), kThreads, 0, st, g, ph, waves, acc, health);
 }
 
 template <typename real, bool GRAV>
@@ -194,7 +201,7 @@ void launchHllcFluxG(const Grid& g, const Phys<real>& ph, const real* stage, con
         dim3 grid((unsigned)((g.S[0] + FT::X - 1) / FT::X),                                                       \
                   (unsigned)(DD == 2 ? (s1 - s0 + FT::Y - 1) / FT::Y : (g.S[1] + FT::Y - 1) / FT::Y),             \
                   (unsigned)(DD == 2 ? 1 : (s1 - s0 + FT::Z - 1) / FT::Z));                                        \
-        hllcFluxTileKernel<real, DD, H, GRAV><<<grid, kThreads, 0, st>>>(g, ph, stage, waves, flux, health, pot,  \
+        launchDependent(hllcFluxTileKernel<real, DD, H, GRAV>, grid, kThreads, 0, st, g, ph, stage, waves, flux, health, pot,  \
                                                                           s0, s1);                                \
     }
         if (hll) {
@@ -202,7 +209,7 @@ void launchHllcFluxG(const Grid& g, const Phys<real>& ph, const real* stage, con
             else T(3, true)
         } else {
             if (g.dim == 2)
-                hllcFluxTileKernelWide<real, GRAV><<<tileGrid<2>(g, s0, s1), kThreads, 0, st>>>(g, ph, stage, waves,
+                launchDependent(hllcFluxTileKernelWide<real, GRAV>, tileGrid<2>(g, s0, s1), kThreads, 0, st, g, ph, stage, waves,
                                                                                                 flux, health, pot, s0,
                                                                                                 s1);
             else T(3, false)
@@ -211,7 +218,7 @@ void launchHllcFluxG(const Grid& g, const Phys<real>& ph, const real* stage, con
         return;
     }
 #define L(DD, H)                                                                                                  \
-    hllcFluxKernel<real, DD, H, GRAV><<<blocksFor(c1 - c0), kThreads, 0, st>>>(g, ph, stage, waves, flux, health, pot, \
+    launchDependent(hllcFluxKernel<real, DD, H, GRAV>, blocksFor(c1 - c0), kThreads, 0, st, g, ph, stage, waves, flux, health, pot, \
                                                                              c0, c1)
     if (hll) {
         if (g.dim == 1) L(1, true);

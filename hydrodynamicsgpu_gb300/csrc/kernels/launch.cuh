@@ -1,0 +1,38 @@
+// launch.cuh -- kernel launches that overlap the start of one kernel with the end of the
+// kernel before it in the stream (programmatic dependent launch).
+//
+// A step is a chain of 10 to 200 kernels, each reading what the one before wrote.  Launched
+// plainly, a kernel starts after the previous grid has drained; here it is launched with
+// programmatic stream serialization, so its blocks take their places as soon as every block
+// of the previous grid is resident or done, and each kernel begins with dependentLaunch():
+// let the next grid start in turn, then wait until the previous grid has completed and its
+// writes are visible.  Nothing is read or written before that wait, so the order of memory
+// operations is that of plain launches.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace hgpu {
+
+__device__ __forceinline__ void dependentLaunch() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// kernel<<<grid, block, smem, st>>>(args...) with that attribute; every kernel launched
+// this way calls dependentLaunch() first
+template <typename... P, typename... A>
+inline void launchDependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace hgpu

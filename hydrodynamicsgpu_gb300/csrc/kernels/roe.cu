@@ -10,6 +10,7 @@
 // roe_cells.cuh (shared with the batched kernels).
 #include "../../../include/hgpu/hgpu.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "reduce.cuh"
 #include "roe_cells.cuh"
 
@@ -36,6 +37,7 @@ template <typename real, int D, bool GRAV>
 __global__ void __launch_bounds__(256) roeBasisKernel(Grid g, Phys<real> ph, const real* __restrict__ state,
                                                      real* __restrict__ basis, int loA, int hiA,
                                                      const real* __restrict__ pot, int slowOff) {
+    dependentLaunch();
     typedef BasisTile<D> T;
     constexpr int HX = T::X + 1, HY = D > 1 ? T::Y + 1 : 1, HZ = D > 2 ? T::Z + 1 : 1;
     __shared__ RoePrim<real, D> prim[HZ * HY * HX];
@@ -47,6 +49,7 @@ __global__ void __launch_bounds__(256) roeBasisKernel(Grid g, Phys<real> ph, con
 template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) roeDtKernel(Grid g, Phys<real> ph, const real* __restrict__ basis,
                                                         unsigned long long* acc, unsigned* health) {
+    dependentLaunch();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long best = ~0ULL;
     bool nan = false;
@@ -63,6 +66,7 @@ template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) roeDeltaQKernel(Grid g, const real* __restrict__ stage,
                                                             const real* __restrict__ basis, real* __restrict__ dq,
                                                             int loA, int hiA, long long c0, long long c1) {
+    dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
     int x, y, z;
@@ -75,6 +79,7 @@ __global__ void __launch_bounds__(kThreads) roeFluxKernel(Grid g, int lim, const
                                                           const real* __restrict__ basis, const real* __restrict__ dq,
                                                           const StepConst<real>* __restrict__ sc,
                                                           real* __restrict__ flux, long long c0, long long c1) {
+    dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
     int x, y, z;
@@ -87,6 +92,7 @@ __global__ void __launch_bounds__(kThreads) roeFluxCorrKernel(Grid g, int lim, c
                                                               const double* __restrict__ dq,
                                                               const StepConst<double>* __restrict__ sc,
                                                               double* __restrict__ flux, long long c0, long long c1) {
+    dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
     int x, y, z;
@@ -98,6 +104,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads) roeFluxXformKernel(Grid g, const double* __restrict__ stage,
                                                                const double* __restrict__ basis,
                                                                double* __restrict__ flux, long long c0, long long c1) {
+    dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
     int x, y, z;
@@ -115,7 +122,7 @@ void launchRoeBasisG(const Grid& g, const Phys<real>& ph, const real* state, rea
                     (unsigned)((g.S[2] + tz - 1) / tz));
     };
     if (g.dim == 1) {
-        roeBasisKernel<real, 1, GRAV><<<grid(BasisTile<1>::X, 1, 1), 256, 0, st>>>(g, ph, state, basis, loA, hiA, pot,
+        launchDependent(roeBasisKernel<real, 1, GRAV>, grid(BasisTile<1>::X, 1, 1), 256, 0, st, g, ph, state, basis, loA, hiA, pot,
                                                                                    0);
         return;
     }
@@ -127,9 +134,9 @@ void launchRoeBasisG(const Grid& g, const Phys<real>& ph, const real* state, rea
     if (slowTiles <= 0) return;
     slow = (unsigned)slowTiles;
     if (g.dim == 2)
-        roeBasisKernel<real, 2, GRAV><<<gr, 256, 0, st>>>(g, ph, state, basis, loA, hiA, pot, slow0);
+        launchDependent(roeBasisKernel<real, 2, GRAV>, gr, 256, 0, st, g, ph, state, basis, loA, hiA, pot, slow0);
     else
-        roeBasisKernel<real, 3, GRAV><<<gr, 256, 0, st>>>(g, ph, state, basis, loA, hiA, pot, slow0);
+        launchDependent(roeBasisKernel<real, 3, GRAV>, gr, 256, 0, st, g, ph, state, basis, loA, hiA, pot, slow0);
 }
 
 // REF: faces along [2, S-2] (res/EulerRoe.cl:27-34, res/Roe.cl:88-95); SEAM: [1, S-1].
@@ -147,9 +154,9 @@ int roeBasisSlowTile(int dim) { return dim == 2 ? BasisTile<2>::Y : dim == 3 ? B
 template <typename real>
 void launchRoeDt(const Grid& g, const Phys<real>& ph, const real* basis, unsigned long long* acc, unsigned* health,
                  cudaStream_t st) {
-    if (g.dim == 1) roeDtKernel<real, 1><<<blocksFor(g.V), kThreads, 0, st>>>(g, ph, basis, acc, health);
-    else if (g.dim == 2) roeDtKernel<real, 2><<<blocksFor(g.V), kThreads, 0, st>>>(g, ph, basis, acc, health);
-    else roeDtKernel<real, 3><<<blocksFor(g.V), kThreads, 0, st>>>(g, ph, basis, acc, health);
+    if (g.dim == 1) launchDependent(roeDtKernel<real, 1>, blocksFor(g.V), kThreads, 0, st, g, ph, basis, acc, health);
+    else if (g.dim == 2) launchDependent(roeDtKernel<real, 2>, blocksFor(g.V), kThreads, 0, st, g, ph, basis, acc, health);
+    else launchDependent(roeDtKernel<real, 3>, blocksFor(g.V), kThreads, 0, st, g, ph, basis, acc, health);
 }
 
 // cells [c0, c1) (c1 < 0: to the end of the grid); whole-grid launches take every cell
@@ -162,9 +169,9 @@ void launchRoeDeltaQ(const Grid& g, const real* stage, const real* basis, real* 
     c1 = rangeEnd(g, c1);
     if (c1 <= c0) return;
     const unsigned b = blocksFor(c1 - c0);
-    if (g.dim == 1) roeDeltaQKernel<real, 1><<<b, kThreads, 0, st>>>(g, stage, basis, dq, loA, hiA, c0, c1);
-    else if (g.dim == 2) roeDeltaQKernel<real, 2><<<b, kThreads, 0, st>>>(g, stage, basis, dq, loA, hiA, c0, c1);
-    else roeDeltaQKernel<real, 3><<<b, kThreads, 0, st>>>(g, stage, basis, dq, loA, hiA, c0, c1);
+    if (g.dim == 1) launchDependent(roeDeltaQKernel<real, 1>, b, kThreads, 0, st, g, stage, basis, dq, loA, hiA, c0, c1);
+    else if (g.dim == 2) launchDependent(roeDeltaQKernel<real, 2>, b, kThreads, 0, st, g, stage, basis, dq, loA, hiA, c0, c1);
+    else launchDependent(roeDeltaQKernel<real, 3>, b, kThreads, 0, st, g, stage, basis, dq, loA, hiA, c0, c1);
 }
 
 template <int LIM>
@@ -172,14 +179,14 @@ void launchRoeFluxSplit(const Grid& g, int limiter, const double* stage, const d
                         const StepConst<double>* sc, double* flux, cudaStream_t st, long long c0, long long c1) {
     const unsigned b = blocksFor(c1 - c0);
     if (g.dim == 1) {
-        roeFluxCorrKernel<1, LIM><<<b, kThreads, 0, st>>>(g, limiter, basis, dq, sc, flux, c0, c1);
-        roeFluxXformKernel<1><<<b, kThreads, 0, st>>>(g, stage, basis, flux, c0, c1);
+        launchDependent(roeFluxCorrKernel<1, LIM>, b, kThreads, 0, st, g, limiter, basis, dq, sc, flux, c0, c1);
+        launchDependent(roeFluxXformKernel<1>, b, kThreads, 0, st, g, stage, basis, flux, c0, c1);
     } else if (g.dim == 2) {
-        roeFluxCorrKernel<2, LIM><<<b, kThreads, 0, st>>>(g, limiter, basis, dq, sc, flux, c0, c1);
-        roeFluxXformKernel<2><<<b, kThreads, 0, st>>>(g, stage, basis, flux, c0, c1);
+        launchDependent(roeFluxCorrKernel<2, LIM>, b, kThreads, 0, st, g, limiter, basis, dq, sc, flux, c0, c1);
+        launchDependent(roeFluxXformKernel<2>, b, kThreads, 0, st, g, stage, basis, flux, c0, c1);
     } else {
-        roeFluxCorrKernel<3, LIM><<<b, kThreads, 0, st>>>(g, limiter, basis, dq, sc, flux, c0, c1);
-        roeFluxXformKernel<3><<<b, kThreads, 0, st>>>(g, stage, basis, flux, c0, c1);
+        launchDependent(roeFluxCorrKernel<3, LIM>, b, kThreads, 0, st, g, limiter, basis, dq, sc, flux, c0, c1);
+        launchDependent(roeFluxXformKernel<3>, b, kThreads, 0, st, g, stage, basis, flux, c0, c1);
     }
 }
 
@@ -193,9 +200,9 @@ void launchRoeFluxLim(const Grid& g, int limiter, const real* stage, const real*
         return;
     }
     const unsigned b = blocksFor(c1 - c0);
-    if (g.dim == 1) roeFluxKernel<real, 1, LIM><<<b, kThreads, 0, st>>>(g, limiter, stage, basis, dq, sc, flux, c0, c1);
-    else if (g.dim == 2) roeFluxKernel<real, 2, LIM><<<b, kThreads, 0, st>>>(g, limiter, stage, basis, dq, sc, flux, c0, c1);
-    else roeFluxKernel<real, 3, LIM><<<b, kThreads, 0, st>>>(g, limiter, stage, basis, dq, sc, flux, c0, c1);
+    if (g.dim == 1) launchDependent(roeFluxKernel<real, 1, LIM>, b, kThreads, 0, st, g, limiter, stage, basis, dq, sc, flux, c0, c1);
+    else if (g.dim == 2) launchDependent(roeFluxKernel<real, 2, LIM>, b, kThreads, 0, st, g, limiter, stage, basis, dq, sc, flux, c0, c1);
+    else launchDependent(roeFluxKernel<real, 3, LIM>, b, kThreads, 0, st, g, limiter, stage, basis, dq, sc, flux, c0, c1);
 }
 
 // the benchmark limiters and the common ones get kernels of their own; the others

@@ -28,6 +28,7 @@
 #include "../../../include/hgpu/hgpu.h"
 #include "combine_cells.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "roe_cells.cuh"
 #include "tma.cuh"
 
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(kThreadsX, kBlocksX)
     roeStageXKernel(Grid g, Phys<double> ph, int lim, const StepConst<double>* __restrict__ sc,
                     const double* __restrict__ stage, const double* __restrict__ basis, double* __restrict__ dX,
                     int loA, int hiA, unsigned* health) {
+    dependentLaunch();
     constexpr int N = 4, NB = RoeRec<2>::NB;
     __shared__ __align__(128) double sS[(kSegX + 4) * N];   // cells [x0 - 2, xEnd + 1]
     __shared__ __align__(16) double sQ[(kSegX + 3) * N];    // Delta-q-tilde, faces [x0 - 1, xEnd + 1]
@@ -156,6 +158,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     roeStageYKernel(Grid g, Phys<double> ph, int lim, const StepConst<double>* __restrict__ sc,
                     const double* __restrict__ basis, const double* __restrict__ dX, CombinePlan<double> plan,
                     const __grid_constant__ CUtensorMap tm, int loA, int hiA, unsigned* health) {
+    dependentLaunch();
     constexpr int N = 4, NB = RoeRec<2>::NB;
     constexpr unsigned kBox = kRows * kRow * sizeof(double);
     extern __shared__ __align__(128) unsigned char smemRaw[];
@@ -292,10 +295,10 @@ void launchFusedLim(const Grid& g, const Phys<double>& ph, int limiter, const St
     const int rows = g.S[1] - 4;
     const int segs = (g.S[0] - 4 + kSegX - 1) / kSegX;
     if (rows > 0 && segs > 0)
-        roeStageXKernel<LIM><<<dim3(segs, rows), kThreadsX, 0, st>>>(g, ph, limiter, sc, stage, basis, dX, loA, hiA,
+        launchDependent(roeStageXKernel<LIM>, dim3(segs, rows), kThreadsX, 0, st, g, ph, limiter, sc, stage, basis, dX, loA, hiA,
                                                                    health);
     dim3 grid((g.S[0] + kCols - 1) / kCols, (g.S[1] + kStrip - 1) / kStrip);
-    roeStageYKernel<LIM><<<grid, kThreads, sizeof(YShared), st>>>(g, ph, limiter, sc, basis, dX, plan, tm, loA, hiA,
+    launchDependent(roeStageYKernel<LIM>, grid, kThreads, sizeof(YShared), st, g, ph, limiter, sc, basis, dX, plan, tm, loA, hiA,
                                                                    health);
 }
 

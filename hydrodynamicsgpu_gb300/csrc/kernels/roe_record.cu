@@ -3,6 +3,7 @@
 // write is bit-identical to the production FP64 flux's (same code, extra stores).
 #include "../../../include/hgpu/hgpu.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "roe_cells.cuh"
 
 namespace hgpu {
@@ -19,6 +20,7 @@ __global__ void __launch_bounds__(kThreads) roeFluxCorrRecordKernel(Grid g, int 
                                                                     const StepConst<double>* __restrict__ sc,
                                                                     double* __restrict__ flux,
                                                                     double* __restrict__ tape) {
+    dependentLaunch();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
     int x, y, z;
@@ -31,6 +33,7 @@ __global__ void __launch_bounds__(kThreads) roeFluxXformRecordKernel(Grid g, con
                                                                      const double* __restrict__ basis,
                                                                      double* __restrict__ flux,
                                                                      double* __restrict__ tape) {
+    dependentLaunch();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
     int x, y, z;
@@ -43,8 +46,8 @@ void launchLim(const Grid& g, int lim, const double* stage, const double* basis,
                const StepConst<double>* sc, double* flux, double* tape, cudaStream_t st) {
     const unsigned blocks = (unsigned)((g.V + kThreads - 1) / kThreads);
 #define L(DD)                                                                                            \
-    roeFluxCorrRecordKernel<DD, LIM><<<blocks, kThreads, 0, st>>>(g, lim, basis, dq, sc, flux, tape);      \
-    roeFluxXformRecordKernel<DD><<<blocks, kThreads, 0, st>>>(g, stage, basis, flux, tape)
+    launchDependent(roeFluxCorrRecordKernel<DD, LIM>, blocks, kThreads, 0, st, g, lim, basis, dq, sc, flux, tape);      \
+    launchDependent(roeFluxXformRecordKernel<DD>, blocks, kThreads, 0, st, g, stage, basis, flux, tape)
     if (g.dim == 1) { L(1); }
     else if (g.dim == 2) { L(2); }
     else { L(3); }
