@@ -48,7 +48,7 @@ HEADERS = ["kernels/fp64ops.cuh", "kernels/common.cuh", "kernels/roe_cells.cuh",
            "kernels/combine_cells.cuh", "kernels/batch.h", "kernels/batch_common.cuh", "host/batch_solver.h", "kernels/roe.cuh", "kernels/reduce.cuh", "kernels/kernels.h", "host/solver.h",
            "kernels/adjoint.h", "host/adjoint.h",
            "kernels/limiter_dual.cuh", "host/fits.h", "kernels/gravity.h", "kernels/health.cuh",
-           "kernels/tma.cuh", "kernels/launch.cuh"]
+           "kernels/tma.cuh", "kernels/launch.cuh", "kernels/cfl.cuh"]
 
 
 def nvcc():

@@ -10,8 +10,6 @@
 
 namespace hgpu {
 
-static const unsigned long long kAccInf = 0x7FF0000000000000ULL;   // the bits of +Inf
-
 RoeAdjoint::RoeAdjoint(const ResolvedConfig& rc, cudaStream_t stream) : rc_(rc), stream_(stream) {
     rc_.grid.check = checkWord();
     if (rc.cfg.solver != HGPU_SOLVER_ROE || rc.cfg.precision != HGPU_FP64 || rc.cfg.compat != HGPU_COMPAT_REF)
@@ -36,11 +34,7 @@ RoeAdjoint::RoeAdjoint(const ResolvedConfig& rc, cudaStream_t stream) : rc_(rc),
     cur_ = DeviceBuffer(sizeof(double) * V * N, true);
     flux_ = DeviceBuffer(sizeof(double) * V * N * D, true);
     sc_ = DeviceBuffer(sizeof(StepConst<double>), true);
-    acc_ = DeviceBuffer(sizeof(unsigned long long), true);
-    {   // the CFL minimum starts from +Inf (every Roe dtBuffer entry is written, Solver.cpp:217-222)
-        const unsigned long long inf = kAccInf;
-        cudaCheck(cudaMemcpy(acc_.get(), &inf, sizeof inf, cudaMemcpyHostToDevice), "dt accumulator init");
-    }
+    acc_ = DeviceBuffer(sizeof(CflAcc), true);
     health_ = DeviceBuffer(sizeof(unsigned), true);
     lamTmp_ = DeviceBuffer(sizeof(double) * V * N, true);
     if (!fe_) {
@@ -93,14 +87,10 @@ void RoeAdjoint::forward(const double* u_n, double dt, Tape& t, double* u_next, 
     launchBoundary<double>(g, methods_, cur, stream_);
     launchRoeBasis<double>(g, ph_, cur, t.basis.as<double>(), 0, stream_);
     if (dtOut) {                                   // Solver::update's CFL dt
-        launchRoeDt<double>(g, ph_, t.basis.as<double>(), acc_.as<unsigned long long>(), health_.as<unsigned>(),
-                            stream_);
-        launchFinalizeDt<double>(ph_, integ_, 0, 0., acc_.as<unsigned long long>(), kAccInf, sc,
-                                 health_.as<unsigned>(), stream_);
+        launchRoeDt<double>(g, ph_, t.basis.as<double>(), integ_, acc_.as<CflAcc>(), sc, stream_);
         cudaCheck(cudaMemcpyAsync(dtOut, &sc->dt_f64, sizeof(double), cudaMemcpyDeviceToDevice, stream_), "record dt");
     } else {
-        launchFinalizeDt<double>(ph_, integ_, 1, dt, acc_.as<unsigned long long>(), 0, sc, health_.as<unsigned>(),
-                                 stream_);
+        launchFixedDt<double>(ph_, integ_, dt, sc, stream_);
     }
     auto stage = [&](int k, const double* in) {
         cudaCheck(cudaMemcpyAsync(t.U[k].get(), in, bytes, cudaMemcpyDeviceToDevice, stream_), "tape stage");

@@ -6,7 +6,6 @@
 #include "solver.h"
 
 #include <algorithm>
-#include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -460,24 +459,6 @@ Solver<real>::~Solver() {
 }
 
 template <typename real>
-unsigned long long Solver<real>::accInit() const {
-    // Roe writes every dtBuffer entry (INFINITY outside the interior); HLLC writes only
-    // the first volume entries, the rest keep their initial max() (Solver.cpp:217-222,
-    // EulerHLLC.cl:135-168), which joins the minimum when dim > 1.
-    bool maxInit = rc.cfg.solver != HGPU_SOLVER_ROE && rc.dim > 1;   // the HLL driver (HLLC and HLL)
-    if (sizeof(real) == 8) {
-        double v = maxInit ? DBL_MAX : std::numeric_limits<double>::infinity();
-        unsigned long long b;
-        std::memcpy(&b, &v, 8);
-        return b;
-    }
-    float v = maxInit ? FLT_MAX : std::numeric_limits<float>::infinity();
-    unsigned int b;
-    std::memcpy(&b, &v, 4);
-    return b;
-}
-
-template <typename real>
 void Solver<real>::init() {                                  // Solver::init (Solver.cpp:48-205)
     equation.reset(new Euler(rc.cfg, rc.dim));
     cudaCheck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -486,8 +467,6 @@ void Solver<real>::init() {                                  // Solver::init (So
     initBuffers();
     if (rc.cfg.integrator == HGPU_INTEGRATOR_FORWARD_EULER) integrator.reset(new ForwardEuler<real>(this));
     else integrator.reset(new RungeKutta<real>(this, rc.cfg.integrator));
-    unsigned long long init = accInit();
-    cudaCheck(cudaMemcpy(dtAcc.get(), &init, sizeof init, cudaMemcpyHostToDevice), "dt accumulator init");
     cudaCheck(cudaDeviceSynchronize(), "init");
 }
 
@@ -496,7 +475,7 @@ void Solver<real>::initBuffers() {                           // Solver::initBuff
     size_t n = (size_t)rc.grid.V * rc.numStates;
     state = DeviceBuffer(sizeof(real) * n, true);
     stepConst = DeviceBuffer(sizeof(StepConst<real>), true);
-    dtAcc = DeviceBuffer(sizeof(unsigned long long), true);
+    dtAcc = DeviceBuffer(sizeof(CflAcc), true);
     healthBuf = DeviceBuffer(sizeof(unsigned), true);
     health = healthBuf.as<unsigned>();
     potential = DeviceBuffer(sizeof(real) * (size_t)rc.grid.V, true);
@@ -584,7 +563,7 @@ double Solver<real>::lastDt() {
 
 template <typename real>
 void Solver<real>::boundaryOn(real* buf) {
-    launch("boundary", rc.dim, [&] { launchBoundary<real>(rc.grid, methods, buf, stream); });
+    launch("boundary", boundaryLaunches(rc.grid), [&] { launchBoundary<real>(rc.grid, methods, buf, stream); });
 }
 
 template <typename real>
@@ -728,7 +707,6 @@ void Solver<real>::hostStep(const void* in, void* out, bool upload, bool downloa
         initStep();
         calcTimestep();
     }
-    finalizeDt(false);
 
     const bool banded = download && integrator->lastCombineWritesState() && !fusedActive() && fluxByPlanes();
     struct Unhook {
@@ -795,11 +773,8 @@ void Solver<real>::hostStep(const void* in, void* out, bool upload, bool downloa
 }
 
 template <typename real>
-void Solver<real>::finalizeDt(bool fixed) {
-    launch("finalize_dt", 1, [&] {
-        launchFinalizeDt<real>(ph, rc.cfg.integrator, fixed ? 1 : 0, rc.cfg.fixed_dt, dtAcc.as<unsigned long long>(),
-                               accInit(), sc(), health, stream);
-    });
+void Solver<real>::fixedDt() {
+    launch("finalize_dt", 1, [&] { launchFixedDt<real>(ph, rc.cfg.integrator, rc.cfg.fixed_dt, sc(), stream); });
 }
 
 template <typename real>
@@ -807,11 +782,8 @@ void Solver<real>::update() {                                // Solver::update (
     this->launches_ = 0;
     boundary();
     initStep();
-    if (rc.cfg.use_fixed_dt) finalizeDt(true);
-    else {
-        calcTimestep();
-        finalizeDt(false);
-    }
+    if (rc.cfg.use_fixed_dt) fixedDt();
+    else calcTimestep();
     step();
     checkState();
 }
@@ -855,8 +827,8 @@ void Roe<real>::initFlux() {                                 // Roe::initFlux (R
 template <typename real>
 void Roe<real>::cflReduce() {
     this->launch("cfl_min_reduce", 1, [&] {
-        launchRoeDt<real>(this->rc.grid, this->ph, basis.template as<real>(),
-                          this->dtAcc.template as<unsigned long long>(), this->health, this->stream);
+        launchRoeDt<real>(this->rc.grid, this->ph, basis.template as<real>(), this->rc.cfg.integrator,
+                          this->dtAcc.template as<CflAcc>(), this->sc(), this->stream);
     });
 }
 
@@ -1007,8 +979,8 @@ void HLL<real>::bandedPrologueWork(int tile0, int tiles, cudaStream_t st) {
 template <typename real>
 void HLL<real>::calcTimestep() {                             // HLL::calcTimestep (HLL.cpp:35-38)
     this->launch("cfl_min_reduce", 1, [&] {
-        launchHllcDt<real>(this->rc.grid, this->ph, waves.template as<real>(),
-                           this->dtAcc.template as<unsigned long long>(), this->health, this->stream);
+        launchHllcDt<real>(this->rc.grid, this->ph, waves.template as<real>(), this->rc.cfg.integrator,
+                           this->dtAcc.template as<CflAcc>(), this->sc(), this->stream);
     });
 }
 

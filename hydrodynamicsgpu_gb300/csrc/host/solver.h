@@ -267,15 +267,14 @@ public:
     std::unique_ptr<Equation> equation;
     std::unique_ptr<Integrator<real>> integrator;
     StepConst<real>* sc() const { return stepConst.as<StepConst<real>>(); }
-    unsigned long long accInit() const;
     int methods[3][2];
 
 protected:
     virtual void initBuffers();
     virtual void initStep() {}
-    virtual void calcTimestep() = 0;        // device-side; leaves the minimum in dtAcc
+    virtual void calcTimestep() = 0;        // device-side; leaves dt and the step's constants in stepConst
     virtual void step() = 0;
-    void finalizeDt(bool fixed);
+    void fixedDt();                         // the step's constants from the fixed dt
     void applyPotential();                  // SelfGravitation::applyPotential (SelfGravitation.cpp:100-124)
     bool potentialLive_ = false;            // useGravity, or a nonzero static potential was given
 

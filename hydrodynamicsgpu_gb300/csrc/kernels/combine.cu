@@ -11,6 +11,8 @@
 //    term before beta term, starting from +0, so every sum is bit-identical;
 //  * findMinTimestep's host read and `dt * cfl` (Solver.cpp:466-516): dt is
 //    finalised on the device, with dt/dx and beta*dt, for the whole step.
+#include <cstring>
+
 #include "combine_cells.cuh"
 #include "kernels.h"
 #include "launch.cuh"
@@ -33,6 +35,8 @@ constexpr int kThreads = 256;
 inline unsigned blocksFor(long long n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
 // ---------------- ghost fill ----------------
+// one axis, one thread a line: axes of 5 cells, where the reference's fill order shows
+// (a ghost is copied from a ghost filled before it)
 template <typename real>
 __global__ void __launch_bounds__(kThreads) boundaryKernel(Grid g, int axis, int N, int mMin, int mMax,
                                                            real* __restrict__ state, long long t0, long long t1) {
@@ -40,6 +44,61 @@ __global__ void __launch_bounds__(kThreads) boundaryKernel(Grid g, int axis, int
     const long long t = t0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= t1) return;
     boundaryLine<real>(g, axis, N, mMin, mMax, state, t);
+}
+
+// one axis, one thread a ghost cell: thread (line t, k-th of the line's four ghosts)
+template <typename real>
+__global__ void __launch_bounds__(kThreads) ghostAxisKernel(Grid g, int axis, int N, int mMin, int mMax,
+                                                            real* __restrict__ state, long long t0, long long t1) {
+    dependentLaunch();
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, t = t0 + i / 4;
+    if (t >= t1) return;
+    const int k = (int)(i & 3), A = axis == 0 ? 1 : 0, S = g.S[axis];
+    const long long nA = g.dim == 1 ? 1 : g.S[A];
+    int c[3] = {0, 0, 0};
+    c[A] = (int)(t % nA);
+    if (g.dim > 1) c[axis == 2 ? 1 : 2] = (int)(t / nA);
+    c[axis] = k < 2 ? k : S - 4 + k;
+    Methods bc = {{{-1, -1}, {-1, -1}, {-1, -1}}};
+    bc.m[axis][0] = mMin;
+    bc.m[axis][1] = mMax;
+    ghostCell<real>(g, N, bc, state, c[0], c[1], c[2]);
+}
+
+// every axis at once, one thread a ghost cell: the ghosts of axis 0 (n0 of them), then those
+// of axis 1 inside axis 0's interior (n1), then those of axis 2 inside both.  The
+// per-line form (a launch an axis, each thread copying its line's ghosts state by state and
+// side by side, every copy after the one before) took 15 us at 133 x 97 and 17 us at
+// 2048^2 for the two launches; this one @B1@ and @B2@ us.
+template <typename real>
+__global__ void __launch_bounds__(kThreads) ghostKernel(Grid g, int N, Methods bc, real* __restrict__ state,
+                                                        long long n0, long long n1, long long n) {
+    dependentLaunch();
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    auto ghost = [](int k, int S) { return k < 2 ? k : S - 4 + k; };
+    int x, y = 0, z = 0;
+    if (i < n0) {
+        x = ghost((int)(i & 3), g.S[0]);
+        i >>= 2;
+        y = (int)(i % g.S[1]);
+        z = (int)(i / g.S[1]);
+    } else if (i < n0 + n1) {
+        i -= n0;
+        const int w = g.S[0] - 4;
+        x = 2 + (int)(i % w);
+        i /= w;
+        y = ghost((int)(i & 3), g.S[1]);
+        z = (int)(i >> 2);
+    } else {
+        i -= n0 + n1;
+        const int w = g.S[0] - 4, h = g.S[1] - 4;
+        x = 2 + (int)(i % w);
+        i /= w;
+        y = 2 + (int)(i % h);
+        z = ghost((int)(i / h), g.S[2]);
+    }
+    ghostCell<real>(g, N, bc, state, x, y, z);
 }
 
 // ---------------- flux divergence + stage combine ----------------
@@ -67,14 +126,11 @@ __global__ void __launch_bounds__(kThreads) alphaOnlyKernel(long long n, int int
 }
 
 template <typename real>
-__global__ void finalizeDtKernel(Phys<real> ph, int integ, int useFixed, double fixedDt, unsigned long long* acc,
-                                 unsigned long long accInit, StepConst<real>* sc) {
+__global__ void fixedDtKernel(Phys<real> ph, int integ, double fixedDt, StepConst<real>* sc) {
     dependentLaunch();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    finalizeOne<real>(ph, integ, useFixed, fixedDt, acc, accInit, sc);
+    finalizeOne<real>(ph, integ, 1, fixedDt, nullptr, 0, sc);
 }
-
-__global__ void resetAccKernel(unsigned long long* acc, unsigned long long v) { dependentLaunch(); *acc = v; }
 
 // Self-gravity pass with ForwardEuler and a zero potential: the (ghost-refreshed)
 // state gets `state + deriv * dt` with deriv == +0 (ForwardEuler.cpp:20-32).
@@ -100,13 +156,31 @@ void launchBoundaryAxis(const Grid& g, const int methods[3][2], real* state, cud
     if (t1 < 0 || t1 > n) t1 = n;
     if (t0 < 0) t0 = 0;
     if (t0 >= t1) return;
-    launchDependent(boundaryKernel<real>, blocksFor(t1 - t0), kThreads, 0, st, g, axis, g.dim + 2, methods[axis][0],
-                                                                   methods[axis][1], state, t0, t1);
+    if (g.S[axis] < 6)
+        launchDependent(boundaryKernel<real>, blocksFor(t1 - t0), kThreads, 0, st, g, axis, g.dim + 2, methods[axis][0],
+                        methods[axis][1], state, t0, t1);
+    else
+        launchDependent(ghostAxisKernel<real>, blocksFor(4 * (t1 - t0)), kThreads, 0, st, g, axis, g.dim + 2,
+                        methods[axis][0], methods[axis][1], state, t0, t1);
+}
+
+int boundaryLaunches(const Grid& g) {
+    for (int a = 0; a < g.dim; ++a)
+        if (g.S[a] < 6) return g.dim;
+    return 1;
 }
 
 template <typename real>
 void launchBoundary(const Grid& g, const int methods[3][2], real* state, cudaStream_t st) {
-    for (int axis = 0; axis < g.dim; ++axis) launchBoundaryAxis<real>(g, methods, state, st, axis, 0, -1);
+    if (boundaryLaunches(g) > 1 || g.S[0] < 6) {   // an axis whose fill order shows: axis by axis
+        for (int axis = 0; axis < g.dim; ++axis) launchBoundaryAxis<real>(g, methods, state, st, axis, 0, -1);
+        return;
+    }
+    Methods bc;
+    std::memcpy(bc.m, methods, sizeof bc.m);
+    const long long n0 = 4ll * g.S[1] * g.S[2], n1 = g.dim > 1 ? 4ll * (g.S[0] - 4) * g.S[2] : 0,
+                    n2 = g.dim > 2 ? 4ll * (g.S[0] - 4) * (g.S[1] - 4) : 0, n = n0 + n1 + n2;
+    launchDependent(ghostKernel<real>, blocksFor(n), kThreads, 0, st, g, g.dim + 2, bc, state, n0, n1, n);
 }
 
 template <typename real>
@@ -134,15 +208,8 @@ void launchZeroAdd(const Grid& g, real* state, const StepConst<real>* sc, cudaSt
 }
 
 template <typename real>
-void launchFinalizeDt(const Phys<real>& ph, int integrator, int useFixed, double fixedDt, unsigned long long* acc,
-                      unsigned long long accInit, StepConst<real>* sc, unsigned* health, cudaStream_t st) {
-    (void)health;
-    launchDependent(finalizeDtKernel<real>, 1, 32, 0, st, ph, integrator, useFixed, fixedDt, acc, accInit, sc);
-}
-
-template <typename real>
-void launchResetAcc(unsigned long long* acc, unsigned long long accInit, cudaStream_t st) {
-    launchDependent(resetAccKernel, 1, 1, 0, st, acc, accInit);
+void launchFixedDt(const Phys<real>& ph, int integrator, double fixedDt, StepConst<real>* sc, cudaStream_t st) {
+    launchDependent(fixedDtKernel<real>, 1, 32, 0, st, ph, integrator, fixedDt, sc);
 }
 
 #define INST(real)                                                                                              \
@@ -153,9 +220,7 @@ void launchResetAcc(unsigned long long* acc, unsigned long long accInit, cudaStr
                                            const StepConst<real>*, cudaStream_t, long long, long long);         \
     template void launchAlphaOnly<real>(const Grid&, int, real*, const StepConst<real>*, cudaStream_t);         \
     template void launchZeroAdd<real>(const Grid&, real*, const StepConst<real>*, cudaStream_t);                \
-    template void launchFinalizeDt<real>(const Phys<real>&, int, int, double, unsigned long long*,              \
-                                         unsigned long long, StepConst<real>*, unsigned*, cudaStream_t);        \
-    template void launchResetAcc<real>(unsigned long long*, unsigned long long, cudaStream_t);
+    template void launchFixedDt<real>(const Phys<real>&, int, double, StepConst<real>*, cudaStream_t);
 INST(double)
 INST(float)
 #undef INST

@@ -46,6 +46,48 @@ __device__ __forceinline__ double kAlphaDev(int i, int m, int k) { return cA[i][
 __device__ __forceinline__ double kBetaDev(int i, int m, int k) { return cB[i][m][k]; }
 }  // namespace
 
+// The boundary methods of a problem ([axis][min, max] of HGPU_BOUNDARY_*).
+struct Methods { int m[3][2]; };
+
+// The coordinate along `axis` that the ghost fill copies coordinate k from (k itself for an
+// interior coordinate or a side without a method), for an axis of S >= 6 cells, where no
+// source is a ghost; `flip`: the copy reflects the normal momentum (MIRROR).
+__device__ __forceinline__ int ghostSource(int k, int S, int mMin, int mMax, bool& flip) {
+    flip = false;
+    const bool low = k < 2, high = k >= S - 2;
+    const int m = low ? mMin : mMax;
+    if (!(low || high) || m < 0) return k;
+    if (m == 0) return low ? k + S - 4 : k - (S - 4);             // periodic
+    flip = m == 1;
+    if (m == 1) return low ? 3 - k : 2 * S - 5 - k;                // mirror
+    return low ? 2 : S - 3;                                        // free flow
+}
+
+// The ghost fill of every axis for one ghost cell: the axes' fills run one after another in
+// the reference (Solver.cpp:448-464), so a cell that is a ghost of several axes ends up with
+// the cell that all its coordinates map to, every MIRROR on the way flipping its axis's
+// momentum.  That source is no ghost of a filled side, so no cell of the pass reads what
+// another writes.  Axes of S >= 6 cells (Grid::dim of them).
+template <typename real>
+__device__ __forceinline__ void ghostCell(const Grid& g, int N, const Methods& bc, real* __restrict__ state, int x,
+                                          int y, int z) {
+    bool f0 = false, f1 = false, f2 = false;
+    const int sx = ghostSource(x, g.S[0], bc.m[0][0], bc.m[0][1], f0);
+    const int sy = g.dim > 1 ? ghostSource(y, g.S[1], bc.m[1][0], bc.m[1][1], f1) : 0;
+    const int sz = g.dim > 2 ? ghostSource(z, g.S[2], bc.m[2][0], bc.m[2][1], f2) : 0;
+    const long long c = x + (long long)g.S[0] * (y + (long long)g.S[1] * z);
+    const long long s = sx + (long long)g.S[0] * (sy + (long long)g.S[1] * sz);
+    if (s == c || !cellOk(g, c) || !cellOk(g, s)) return;
+    const bool flip[3] = {f0, f1, f2};
+    real v[5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j)
+        if (j < N) v[j] = state[(long long)N * s + j];
+#pragma unroll
+    for (int j = 0; j < 5; ++j)
+        if (j < N) state[(long long)N * c + j] = j >= 1 && j <= 3 && j <= g.dim && flip[j - 1] ? -v[j] : v[j];
+}
+
 // One ghost line of the boundary pass along `axis` (thread = transverse line t):
 // every state, min side then max side.  In 1D the reference's Mirror/Reflect/FreeFlow
 // kernels have no range guard and only work-item 0 addresses the buffer; that

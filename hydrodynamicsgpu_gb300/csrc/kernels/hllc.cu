@@ -10,10 +10,14 @@
 // momentum components swapped back once more, exactly as the reference buffer does.
 // With `hll` the same launches run EulerHLL (res/EulerHLL.cl): Davis-bounded wave
 // speeds and the two-state HLL flux; its timestep kernel is HLLC's.
+#include <algorithm>
+#include <cstring>
+#include <limits>
+
 #include "hllc_cells.cuh"
 #include "kernels.h"
 #include "launch.cuh"
-#include "reduce.cuh"
+#include "cfl.cuh"
 
 namespace hgpu {
 namespace {
@@ -33,20 +37,29 @@ __global__ void __launch_bounds__(kThreads) hllcWaveKernel(Grid g, Phys<real> ph
     hllcWaveCell<real, D, HLL, GRAV>(g, ph, gq, state, waves, c, x, y, z, pot);
 }
 
+// blocks of the CFL kernels: a few per SM (152), each over a strided share of the cells, so
+// that the accumulator sees thousands of atomics, not one per 256 cells
+inline unsigned cflBlocks(long long n) { return std::min(blocksFor(n), 152u * 8u); }
+
 template <typename real, int D>
-__global__ void __launch_bounds__(kThreads) hllcDtKernel(Grid g, Phys<real> ph, const real* __restrict__ waves,
-                                                         unsigned long long* acc, unsigned* health) {
+__global__ void __launch_bounds__(kThreads) hllcDtKernel(Grid g, Phys<real> ph, const real* __restrict__ waves, int integ,
+                                                        unsigned long long accInit, CflAcc* acc, StepConst<real>* sc) {
     dependentLaunch();
-    long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long best = ~0ULL;
-    bool nan = false;
-    if (c < g.V) {
+    unsigned long long s[D] = {};
+    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < g.V;
+         c += (long long)gridDim.x * blockDim.x) {
         int x, y, z;
         cellCoords(g, c, x, y, z);
-        best = hllcDtCell<real, D>(g, ph, waves, c, x, y, z, nan);
+        if (!inRange(g, x, y, z, 2, 1)) continue;
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            if (!cellOk(g, c) || !cellOk(g, c + g.step[a])) continue;
+            const unsigned long long b = realBits((real)fabs(hllcSpeed<real>(g, waves, c, a)));
+            s[a] = b > s[a] ? b : s[a];
+        }
     }
-    if (nan) atomicOr(health, HEALTH_NONFINITE_DT);
-    blockMinToGlobal(best, acc);
+    blockMaxSpeeds<D>(s, acc);
+    finishCfl<real, D, false>(ph, integ, accInit, acc, sc);
 }
 
 template <typename real, int D, bool HLL, bool GRAV>
@@ -179,11 +192,17 @@ void launchHllcWaves(const Grid& g, const Phys<real>& ph, const real* state, rea
 }
 
 template <typename real>
-void launchHllcDt(const Grid& g, const Phys<real>& ph, const real* waves, unsigned long long* acc, unsigned* health,
-                  cudaStream_t st) {
-    if (g.dim == 1) launchDependent(hllcDtKernel<real, 1>, blocksFor(g.V), kThreads, 0, st, g, ph, waves, acc, health);
-    else if (g.dim == 2) launchDependent(hllcDtKernel<real, 2>, blocksFor(g.V), kThreads, 0, st, g, ph, waves, acc, health);
-    else launchDependent(hllcDtKernel<real, 3>, blocksFor(g.V), kThreads, 0, st, g, ph, waves, acc, health);
+void launchHllcDt(const Grid& g, const Phys<real>& ph, const real* waves, int integrator, CflAcc* acc,
+                 StepConst<real>* sc, cudaStream_t st) {
+    // the first V entries of the reference's buffer are written; with dim > 1 the rest keep
+    // their initial max() (Solver.cpp:217-222, EulerHLLC.cl:135-168) and join the minimum
+    const real top = g.dim > 1 ? std::numeric_limits<real>::max() : std::numeric_limits<real>::infinity();
+    unsigned long long accInit = 0;
+    std::memcpy(&accInit, &top, sizeof top);
+    const unsigned b = cflBlocks(g.V);
+    if (g.dim == 1) launchDependent(hllcDtKernel<real, 1>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc);
+    else if (g.dim == 2) launchDependent(hllcDtKernel<real, 2>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc);
+    else launchDependent(hllcDtKernel<real, 3>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc);
 }
 
 template <typename real, bool GRAV>
@@ -242,7 +261,7 @@ void launchHllcFlux(const Grid& g, const Phys<real>& ph, const real* stage, cons
 #define INST(real)                                                                                                \
     template void launchHllcWaves<real>(const Grid&, const Phys<real>&, const real*, real*, int, cudaStream_t,    \
                                         const real*, long long, long long);                                       \
-    template void launchHllcDt<real>(const Grid&, const Phys<real>&, const real*, unsigned long long*, unsigned*, \
+    template void launchHllcDt<real>(const Grid&, const Phys<real>&, const real*, int, CflAcc*, StepConst<real>*, \
                                      cudaStream_t);                                                               \
     template void launchHllcFlux<real>(const Grid&, const Phys<real>&, const real*, const real*, real*, unsigned*, \
                                        int, cudaStream_t, const real*, long long, long long);

@@ -167,6 +167,14 @@ __device__ __forceinline__ void hllcWaveCell(const Grid& g, const Phys<real>& ph
     if (D > 2) waveFace<real, D, (D > 2 ? 2 : 0), GRAV>(g, ph, gq, state, waves, c, pot);
 }
 
+// the wave speed difference of cell c along `side`: max(0, sr(face c)) - min(0, sl(face c+1))
+template <typename real>
+__device__ __forceinline__ real hllcSpeed(const Grid& g, const real* __restrict__ waves, long long c, int side) {
+    const real srHere = waves[((long long)side * 2 + 1) * g.V + c];
+    const real slNext = waves[((long long)side * 2 + 0) * g.V + c + g.step[side]];
+    return fmaxLibm((real)0., srHere) - fminLibm((real)0., slNext);
+}
+
 // cell timestep (EulerHLLC.cl:135-168): cells in [2, S-2], min over sides of
 // dx / (max(0, sr(face c)) - min(0, sl(face c+1))); INFINITY elsewhere
 template <typename real, int D>
@@ -178,11 +186,7 @@ __device__ __forceinline__ unsigned long long hllcDtCell(const Grid& g, const Ph
 #pragma unroll
         for (int side = 0; side < D; ++side) {
             if (!cellOk(g, c) || !cellOk(g, c + g.step[side])) continue;
-            real srHere = waves[((long long)side * 2 + 1) * g.V + c];
-            real slNext = waves[((long long)side * 2 + 0) * g.V + c + g.step[side]];
-            real minLambda = (real)fminLibm(0., (double)slNext);
-            real maxLambda = (real)fmaxLibm(0., (double)srHere);
-            real dum = divI(ph.dx[side], maxLambda - minLambda);
+            real dum = divI(ph.dx[side], hllcSpeed<real>(g, waves, c, side));
             if (isNaNBits(dum)) nan = true;
             result = fminLibm(result, dum);
         }

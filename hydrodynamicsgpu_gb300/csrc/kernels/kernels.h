@@ -40,6 +40,7 @@ struct CombinePlan {
 // ---- boundary.cu ----
 template <typename real>
 void launchBoundary(const Grid& g, const int methods[3][2], real* state, cudaStream_t st);
+int boundaryLaunches(const Grid& g);   // the kernels launchBoundary launches
 // the ghost fill along one axis over its transverse lines [t0, t1) (line t of axis a
 // addresses the cell with c[A] + S[A] * c[B] = t, A < B the other two axes)
 long long boundaryLines(const Grid& g, int axis);
@@ -54,11 +55,15 @@ template <typename real>
 void launchAlphaOnly(const Grid& g, int integrator, real* state, const StepConst<real>* sc, cudaStream_t st);
 template <typename real>
 void launchZeroAdd(const Grid& g, real* state, const StepConst<real>* sc, cudaStream_t st);
+// The CFL reduction of a step: the largest wave speed difference of each axis (IEEE bits)
+// and the count of finished blocks, all zero between steps (cfl.cuh).
+struct CflAcc {
+    unsigned long long speed[3];
+    unsigned done;
+};
+// the step's constants from a given dt
 template <typename real>
-void launchFinalizeDt(const Phys<real>& ph, int integrator, int useFixed, double fixedDt, unsigned long long* acc,
-                      unsigned long long accInit, StepConst<real>* sc, unsigned* health, cudaStream_t st);
-template <typename real>
-void launchResetAcc(unsigned long long* acc, unsigned long long accInit, cudaStream_t st);
+void launchFixedDt(const Phys<real>& ph, int integrator, double fixedDt, StepConst<real>* sc, cudaStream_t st);
 
 // ---- roe.cu ----
 // pot: the gravitational potential (V values), or null for a zero potential.  In 2D
@@ -69,8 +74,9 @@ void launchRoeBasis(const Grid& g, const Phys<real>& ph, const real* state, real
                     const real* pot = nullptr, int slow0 = 0, int slowTiles = -1);
 int roeBasisSlowTile(int dim);
 template <typename real>
-void launchRoeDt(const Grid& g, const Phys<real>& ph, const real* basis, unsigned long long* acc, unsigned* health,
-                 cudaStream_t st);
+// the step's CFL timestep and constants into sc (acc: zero before and after)
+void launchRoeDt(const Grid& g, const Phys<real>& ph, const real* basis, int integrator, CflAcc* acc,
+                 StepConst<real>* sc, cudaStream_t st);
 template <typename real>
 // cells [c0, c1) only (c1 < 0: to the end of the grid)
 void launchRoeDeltaQ(const Grid& g, const real* stage, const real* basis, real* dq, int seam, cudaStream_t st,
@@ -87,8 +93,8 @@ template <typename real>
 void launchHllcWaves(const Grid& g, const Phys<real>& ph, const real* state, real* waves, int hll, cudaStream_t st,
                      const real* pot = nullptr, long long c0 = 0, long long c1 = -1);
 template <typename real>
-void launchHllcDt(const Grid& g, const Phys<real>& ph, const real* waves, unsigned long long* acc, unsigned* health,
-                  cudaStream_t st);
+void launchHllcDt(const Grid& g, const Phys<real>& ph, const real* waves, int integrator, CflAcc* acc,
+                  StepConst<real>* sc, cudaStream_t st);
 template <typename real>
 void launchHllcFlux(const Grid& g, const Phys<real>& ph, const real* stage, const real* waves, real* flux,
                     unsigned* health, int hll, cudaStream_t st, const real* pot = nullptr, long long c0 = 0,

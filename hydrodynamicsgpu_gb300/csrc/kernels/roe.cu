@@ -8,10 +8,14 @@
 // entry) instead of two dense N x N matrices, and it is computed once per step
 // from u^n exactly as the reference does (Roe.cpp:82-92).  The bodies live in
 // roe_cells.cuh (shared with the batched kernels).
+#include <algorithm>
+#include <cstring>
+#include <limits>
+
 #include "../../../include/hgpu/hgpu.h"
 #include "kernels.h"
 #include "launch.cuh"
-#include "reduce.cuh"
+#include "cfl.cuh"
 #include "roe_cells.cuh"
 
 namespace hgpu {
@@ -46,20 +50,29 @@ __global__ void __launch_bounds__(256) roeBasisKernel(Grid g, Phys<real> ph, con
                                 T::Z, prim, pot);
 }
 
+// blocks of the CFL kernels: a few per SM (152), each over a strided share of the cells, so
+// that the accumulator sees thousands of atomics, not one per 256 cells
+inline unsigned cflBlocks(long long n) { return std::min(blocksFor(n), 152u * 8u); }
+
 template <typename real, int D>
-__global__ void __launch_bounds__(kThreads) roeDtKernel(Grid g, Phys<real> ph, const real* __restrict__ basis,
-                                                        unsigned long long* acc, unsigned* health) {
+__global__ void __launch_bounds__(kThreads) roeDtKernel(Grid g, Phys<real> ph, const real* __restrict__ basis, int integ,
+                                                        unsigned long long accInit, CflAcc* acc, StepConst<real>* sc) {
     dependentLaunch();
-    long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long best = ~0ULL;
-    bool nan = false;
-    if (c < g.V) {
+    unsigned long long s[D] = {};
+    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < g.V;
+         c += (long long)gridDim.x * blockDim.x) {
         int x, y, z;
         cellCoords(g, c, x, y, z);
-        best = roeDtCell<real, D>(g, ph, basis, c, x, y, z, nan);
+        if (!inRange(g, x, y, z, 2, 2)) continue;
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            if (!cellOk(g, c) || !cellOk(g, c + g.step[a])) continue;
+            const unsigned long long b = realBits(roeSpeed<real, D>(g, basis, c, a));
+            s[a] = b > s[a] ? b : s[a];
+        }
     }
-    if (nan) atomicOr(health, HEALTH_NONFINITE_DT);
-    blockMinToGlobal(best, acc);
+    blockMaxSpeeds<D>(s, acc);
+    finishCfl<real, D, true>(ph, integ, accInit, acc, sc);
 }
 
 template <typename real, int D>
@@ -152,11 +165,15 @@ void launchRoeBasis(const Grid& g, const Phys<real>& ph, const real* state, real
 int roeBasisSlowTile(int dim) { return dim == 2 ? BasisTile<2>::Y : dim == 3 ? BasisTile<3>::Z : 1; }
 
 template <typename real>
-void launchRoeDt(const Grid& g, const Phys<real>& ph, const real* basis, unsigned long long* acc, unsigned* health,
-                 cudaStream_t st) {
-    if (g.dim == 1) launchDependent(roeDtKernel<real, 1>, blocksFor(g.V), kThreads, 0, st, g, ph, basis, acc, health);
-    else if (g.dim == 2) launchDependent(roeDtKernel<real, 2>, blocksFor(g.V), kThreads, 0, st, g, ph, basis, acc, health);
-    else launchDependent(roeDtKernel<real, 3>, blocksFor(g.V), kThreads, 0, st, g, ph, basis, acc, health);
+void launchRoeDt(const Grid& g, const Phys<real>& ph, const real* basis, int integrator, CflAcc* acc,
+                 StepConst<real>* sc, cudaStream_t st) {
+    const real top = std::numeric_limits<real>::infinity();   // outside the interior the reference's buffer holds INFINITY
+    unsigned long long accInit = 0;
+    std::memcpy(&accInit, &top, sizeof top);
+    const unsigned b = cflBlocks(g.V);
+    if (g.dim == 1) launchDependent(roeDtKernel<real, 1>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc);
+    else if (g.dim == 2) launchDependent(roeDtKernel<real, 2>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc);
+    else launchDependent(roeDtKernel<real, 3>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc);
 }
 
 // cells [c0, c1) (c1 < 0: to the end of the grid); whole-grid launches take every cell
@@ -229,7 +246,7 @@ void launchRoeFlux(const Grid& g, int limiter, const real* stage, const real* ba
 #define INST(real)                                                                                              \
     template void launchRoeBasis<real>(const Grid&, const Phys<real>&, const real*, real*, int, cudaStream_t,    \
                                        const real*, int, int);                                                  \
-    template void launchRoeDt<real>(const Grid&, const Phys<real>&, const real*, unsigned long long*, unsigned*, \
+    template void launchRoeDt<real>(const Grid&, const Phys<real>&, const real*, int, CflAcc*, StepConst<real>*, \
                                     cudaStream_t);                                                             \
     template void launchRoeDeltaQ<real>(const Grid&, const real*, const real*, real*, int, cudaStream_t,        \
                                         long long, long long);                                                  \

@@ -76,6 +76,16 @@ __device__ __forceinline__ void roeBasisTile(const Grid& g, const Phys<real>& ph
     __syncthreads();
 }
 
+// The wave speed difference of interior cell c along `side` (res/Roe.cl:4-65):
+// |max(0, lambda_max(face c)) - min(0, lambda_min(face c+1))|
+template <typename real, int D>
+__device__ __forceinline__ real roeSpeed(const Grid& g, const real* __restrict__ basis, long long c, int side) {
+    typedef RoeRec<D> R_;
+    const real lamMax = basis[((long long)side * R_::NB + R_::LAME) * g.V + c];
+    const real lamMin = basis[((long long)side * R_::NB + R_::LAM0) * g.V + c + g.step[side]];
+    return fabs(fmaxLibm((real)0., lamMax) - fminLibm((real)0., lamMin));
+}
+
 // Cell timestep of one cell, as its minimum over axes in IEEE bits (res/Roe.cl:4-65):
 // interior cells dx / (|max(0, lambda_max(face c)) - min(0, lambda_min(face c+1))| + 1e-9),
 // others INFINITY.
@@ -83,17 +93,12 @@ template <typename real, int D>
 __device__ __forceinline__ unsigned long long roeDtCell(const Grid& g, const Phys<real>& ph,
                                                         const real* __restrict__ basis, long long c, int x, int y,
                                                         int z, bool& nan) {
-    typedef RoeRec<D> R_;
     if (!inRange(g, x, y, z, 2, 2)) return realBits((real)INFINITY);
     unsigned long long best = ~0ULL;
 #pragma unroll
     for (int side = 0; side < D; ++side) {
         if (!cellOk(g, c) || !cellOk(g, c + g.step[side])) continue;
-        real lamMax = basis[((long long)side * R_::NB + R_::LAME) * g.V + c];
-        real lamMin = basis[((long long)side * R_::NB + R_::LAM0) * g.V + c + g.step[side]];
-        real maxLambda = fmaxLibm((real)0., lamMax);
-        real minLambda = fminLibm((real)0., lamMin);
-        real dum = (real)divI((double)ph.dx[side], (double)fabs(maxLambda - minLambda) + 1e-9);
+        real dum = (real)divI((double)ph.dx[side], (double)roeSpeed<real, D>(g, basis, c, side) + 1e-9);
         if (dum != dum) nan = true;
         unsigned long long b = realBits(dum);
         best = b < best ? b : best;
