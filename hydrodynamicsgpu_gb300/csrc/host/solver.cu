@@ -217,6 +217,7 @@ ResolvedConfig resolveConfig(const hgpu_config& cfg) {
     g.step[0] = 1;
     g.step[1] = cfg.size[0];
     g.step[2] = (long long)cfg.size[0] * cfg.size[1];
+    for (int i = 0; i < 2; ++i) g.inv[i] = (unsigned)std::min<long long>(0xFFFFFFFFll, (1ll << 32) / cfg.size[i]);
     g.V = (long long)cfg.size[0] * cfg.size[1] * cfg.size[2];
     return rc;
 }

@@ -76,6 +76,16 @@ __device__ __forceinline__ double fmaxLibm(double x, double y) { return selectD(
 __device__ __forceinline__ double plusMinusOne(bool c) {
     return fromBits(c ? 0x3FF0000000000000LL : (long long)0xBFF0000000000000ULL);
 }
+// fmax(0, x) and fmin(0, x), the sign of a zero result aside (NaN gives 0), on the words:
+// through fmaxLibm / fminLibm with a constant 0 the compiler issues FP64 compares
+__device__ __forceinline__ double positivePart(double x) {
+    return selectD(__double2hiint(x) < 0 || isNaNBits(x), 0., x);
+}
+__device__ __forceinline__ double negativePart(double x) {
+    return selectD(__double2hiint(x) >= 0 || isNaNBits(x), 0., x);
+}
+__device__ __forceinline__ float positivePart(float x) { return x > 0.f ? x : 0.f; }
+__device__ __forceinline__ float negativePart(float x) { return x < 0.f ? x : 0.f; }
 // x <= 0 (-0 and +0 included, NaN false) and a <= b, on the words / bit patterns
 __device__ __forceinline__ bool leZero(double x) { return isZeroBits(x) || (__double2hiint(x) < 0 && !isNaNBits(x)); }
 __device__ __forceinline__ bool leZero(float x) { return x <= 0.f; }

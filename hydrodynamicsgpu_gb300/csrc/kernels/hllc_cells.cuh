@@ -172,7 +172,7 @@ template <typename real>
 __device__ __forceinline__ real hllcSpeed(const Grid& g, const real* __restrict__ waves, long long c, int side) {
     const real srHere = waves[((long long)side * 2 + 1) * g.V + c];
     const real slNext = waves[((long long)side * 2 + 0) * g.V + c + g.step[side]];
-    return fmaxLibm((real)0., srHere) - fminLibm((real)0., slNext);
+    return positivePart(srHere) - negativePart(slNext);
 }
 
 // cell timestep (EulerHLLC.cl:135-168): cells in [2, S-2], min over sides of

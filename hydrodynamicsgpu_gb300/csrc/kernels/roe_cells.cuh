@@ -83,7 +83,7 @@ __device__ __forceinline__ real roeSpeed(const Grid& g, const real* __restrict__
     typedef RoeRec<D> R_;
     const real lamMax = basis[((long long)side * R_::NB + R_::LAME) * g.V + c];
     const real lamMin = basis[((long long)side * R_::NB + R_::LAM0) * g.V + c + g.step[side]];
-    return fabs(fmaxLibm((real)0., lamMax) - fminLibm((real)0., lamMin));
+    return fabs(positivePart(lamMax) - negativePart(lamMin));
 }
 
 // Cell timestep of one cell, as its minimum over axes in IEEE bits (res/Roe.cl:4-65):
