@@ -109,9 +109,10 @@ void RoeAdjoint::forward(const double* u_n, double dt, Tape& t, double* u_next, 
     } else {
         for (int k = 0; k < stages_; ++k) {
             stage(k, plans_.plans[k].slot[plans_.inputSlot[k]]);
-            launchDerivCombine<double>(g, ph_, flux_.as<double>(), plans_.plans[k], sc, stream_);
+            CombinePlan<double> plan = plans_.plans[k];
+            if (k == stages_ - 1 && !alphaBinary_) plan.alphaAfter = integ_;   // the self-gravity pass
+            launchDerivCombine<double>(g, ph_, flux_.as<double>(), plan, sc, stream_);
         }
-        if (!alphaBinary_) launchAlphaOnly<double>(g, integ_, cur, sc, stream_);
     }
     if (u_next && u_next != cur)
         cudaCheck(cudaMemcpyAsync(u_next, cur, bytes, cudaMemcpyDeviceToDevice, stream_), "adjoint output");

@@ -388,30 +388,35 @@ template <typename real>
 void RungeKutta<real>::integrate(const std::function<void(real* stage)>& computeFlux) {
     Solver<real>* s = this->solver;
     for (int k = 0; k < order_; ++k) {
-        real* in = plans_[k].slot[inputSlot_[k]];
+        CombinePlan<real> plan = plans_[k];
+        real* in = plan.slot[inputSlot_[k]];
+        // the last combine also does the zero-potential self-gravity pass (integrateZeroDeriv)
+        if (k == order_ - 1 && !alphaIsBinary_ && !s->potentialLive()) plan.alphaAfter = tableau_;
         if (k == order_ - 1 && this->lastStage) {
-            this->lastStage(in, plans_[k]);
+            this->lastStage(in, plan);
             continue;
         }
         computeFlux(in);
         s->launch("flux_divergence_combine", 1, [&] {
-            launchDerivCombine<real>(s->rc.grid, s->ph, s->flux.template as<real>(), plans_[k], s->sc(), s->stream);
+            launchDerivCombine<real>(s->rc.grid, s->ph, s->flux.template as<real>(), plan, s->sc(), s->stream);
         });
     }
+    zeroDerivDone_ = true;
 }
 
 // the same stages; plans_[k] never writes the slot stage k reads (buildStagePlans)
 template <typename real>
 void RungeKutta<real>::integrateFused(const std::function<void(real*, const CombinePlan<real>&)>& stageKernel) {
     for (int k = 0; k < order_; ++k) stageKernel(plans_[k].slot[inputSlot_[k]], plans_[k]);
+    zeroDerivDone_ = false;
 }
 
 template <typename real>
 void RungeKutta<real>::integrateZeroDeriv() {
     // With every deriv +0 the stage states are alpha-combinations of u^n.  For
     // tableaus whose alphas are all 0 or 1 that is u^n itself (the step leaves no -0
-    // in the state), so nothing runs.
-    if (alphaIsBinary_) return;
+    // in the state), so nothing runs; for the others integrate()'s last combine did it.
+    if (alphaIsBinary_ || zeroDerivDone_) return;
     Solver<real>* s = this->solver;
     s->launch("gravity_pass", 1, [&] {
         launchAlphaOnly<real>(s->rc.grid, tableau_, s->state.template as<real>(), s->sc(), s->stream);

@@ -158,10 +158,11 @@ public:
     void integrateGravity() override;
     int order() const override { return order_; }
     int extraBuffers() const override { return nslots_; }
-    bool lastCombineWritesState() const override { return alphaIsBinary_; }
+    bool lastCombineWritesState() const override { return true; }
 private:
     int tableau_, order_, nslots_ = 0;
     bool alphaIsBinary_ = true;
+    bool zeroDerivDone_ = false;             // integrate() folded the self-gravity pass into its last combine
     std::vector<CombinePlan<real>> plans_;   // one per stage
     std::vector<int> inputSlot_;             // stage k reads u^(k) from this slot
     std::vector<bool> callbackK_;            // the reference calls back at stage k (a nonzero beta in column k)

@@ -141,10 +141,14 @@ __device__ __forceinline__ double mulZ(double x, double y) {
 }
 __device__ __forceinline__ float mulZ(float x, float y) { return x * y; }
 
-// FLATD: the deriv's products by mulZ (the batched kernels, whose states are mostly flat)
-template <typename real, int D, bool FLATD = false>
+// FLATD: the deriv's products by mulZ (the batched kernels, whose states are mostly flat).
+// POST: the new state (the row that slot 0 gets) goes through the self-gravity pass with a
+// zero potential, of the tableau plan.alphaAfter, before it is stored.
+template <typename real, int D, bool FLATD = false, bool POST = false>
 __device__ __forceinline__ void combinePlanCell(const real* d, const CombinePlan<real>& plan,
                                                 const StepConst<real>& sc, long long c, long long off);
+template <typename real>
+__device__ __forceinline__ real alphaOnlyElem(int integ, real u0, const StepConst<real>& sc);
 
 // Flux divergence and Runge-Kutta combine of one cell (res/CalcFluxDeriv.cl:7-44 and
 // the multAdd chain).  `off` is the cell offset of this grid inside the slot arrays
@@ -152,7 +156,7 @@ __device__ __forceinline__ void combinePlanCell(const real* d, const CombinePlan
 // deltaFlux / dx with dx's reciprocal bits from the host (quotBy): KH 2048^2 FP64 237 us
 // a launch, 286 us with the x quotients by Markstein's two FMAs on the FP64 unit and the
 // rest by divI.
-template <typename real, int D, bool FLATD = false>
+template <typename real, int D, bool FLATD = false, bool POST = false>
 __device__ __forceinline__ void derivCombineCell(const Grid& g, const Phys<real>& ph, const real* __restrict__ flux,
                                                  const CombinePlan<real>& plan, const StepConst<real>& sc,
                                                  long long c, int x, int y, int z, long long off) {
@@ -178,12 +182,12 @@ __device__ __forceinline__ void derivCombineCell(const Grid& g, const Phys<real>
 #pragma unroll
         for (int j = 0; j < N; ++j) d[j] = (real)0.;
     }
-    combinePlanCell<real, D, FLATD>(d, plan, sc, c, off);
+    combinePlanCell<real, D, FLATD, POST>(d, plan, sc, c, off);
 }
 
 // The integrator's use of one cell's deriv d: ForwardEuler's state += deriv * dt, or
 // this stage's column of the Runge-Kutta rows (see combine.cu).
-template <typename real, int D, bool FLATD>
+template <typename real, int D, bool FLATD, bool POST>
 __device__ __forceinline__ void combinePlanCell(const real* d, const CombinePlan<real>& plan,
                                                 const StepConst<real>& sc, long long c, long long off) {
     const int N = D + 2;
@@ -224,6 +228,10 @@ __device__ __forceinline__ void combinePlanCell(const real* d, const CombinePlan
             }
         }
         real* o_ = plan.slot[op.out] + (long long)N * (off + c);
+        if (POST && op.out == 0) {
+#pragma unroll
+            for (int j = 0; j < N; ++j) v[j] = alphaOnlyElem<real>(plan.alphaAfter, v[j], sc);
+        }
 #pragma unroll
         for (int j = 0; j < N; ++j) o_[j] = v[j];
     }
@@ -248,23 +256,49 @@ __device__ __forceinline__ void finalizeOne(const Phys<real>& ph, int integ, int
         for (int k = 0; k < 4; ++k) sc->coef[m][k] = (real)kBetaDev(integ, m, k) * dt;
 }
 
-// self-gravity pass with a zero potential and a Runge-Kutta integrator, one element
+// r + t without the FP64 unit where that is exact on the bits: t a zero (r is never -0
+// here), or r and t the same normal number whose double is normal
+static __device__ __noinline__ double addNative(double r, double t) { return r + t; }
+__device__ __forceinline__ double addEqual(double r, double t) {
+    if (isZeroBits(t)) return r;
+    const unsigned e = (unsigned)__double2hiint(r) & 0x7FF00000u;
+    if (bitsOf(r) == bitsOf(t) && e - 0x00100000u < 0x7FD00000u)
+        return __hiloint2double(__double2hiint(r) + 0x00100000, __double2loint(r));
+    return addNative(r, t);
+}
+__device__ __forceinline__ float addEqual(float r, float t) { return r + t; }
+
+// The self-gravity pass with a zero potential and a Runge-Kutta integrator, one element:
+// every deriv is +0, so the stages are alpha combinations of u0 (the 0 * beta dt terms are
+// zeros and change no sum that starts from +0; with a dt that is not finite they are NaN
+// and the terms are kept).  Row by row as the integrator adds them; two equal halves
+// (RungeKutta2TVD) and zeros need no addition.
 template <typename real>
 __device__ __forceinline__ real alphaOnlyElem(int integ, real u0, const StepConst<real>& sc) {
     const int order = kOrderDev(integ);
+    const bool keepZeros = !finiteBits(sc.dt);
     real u[5];
     u[0] = u0;
-    for (int s = 1; s <= order; ++s) {
-        real r = 0;
-        bool empty = true;
+    real out = u0;
+#pragma unroll
+    for (int s = 1; s <= 4; ++s) {
+        if (s > order) break;
+        real r = (real)0;
+#pragma unroll
         for (int k = 0; k < s; ++k) {
-            double a = kAlphaDev(integ, s - 1, k), b = kBetaDev(integ, s - 1, k);
-            if (a != 0) { real t = u[k] * (real)a; r = empty ? zfix(t) : r + t; empty = false; }
-            if (b != 0) { real t = (real)0. * sc.coef[s - 1][k]; r = empty ? zfix(t) : r + t; empty = false; }
+            const double a = kAlphaDev(integ, s - 1, k);
+            // (the tests on the bits: compares of doubles issue to the FP64 unit)
+            if (bitsOf(a) != 0) {
+                const real t = bitsOf(a) == 0x3FF0000000000000LL   ? u[k]
+                               : bitsOf(a) == 0x3FE0000000000000LL ? halfOf(u[k])
+                                                                   : mulZ(u[k], (real)a);
+                r = k == 0 ? zfix(t) : addEqual(r, t);
+            }
+            if (keepZeros && bitsOf(kBetaDev(integ, s - 1, k)) != 0) r = r + (real)0. * sc.coef[s - 1][k];
         }
-        u[s] = r;
+        out = u[s] = r;
     }
-    return u[order];
+    return out;
 }
 
 }  // namespace hgpu

@@ -37,14 +37,15 @@ __device__ __forceinline__ bool isZeroBits(double x) {
 __device__ __forceinline__ bool geZero(float x) { return x >= 0.f; }
 __device__ __forceinline__ bool isZeroBits(float x) { return (__float_as_int(x) & 0x7FFFFFFF) == 0; }
 
-// .5 * x exactly: decrement the exponent of a normal x whose half is normal.  The
-// rare other operands (zero, subnormal, Inf, NaN) take the FP64 unit out of line, so
-// the compiler cannot issue that product for every operand and select.
+// .5 * x exactly: decrement the exponent of a normal x whose half is normal; a zero, an
+// infinity or a NaN is its own half.  The rare other operands (subnormal, or with a
+// subnormal half) take the FP64 unit out of line, so the compiler cannot issue that
+// product for every operand and select.
 static __device__ __noinline__ double halfNative(double x) { return x * .5; }
 __device__ __forceinline__ double halfOf(double x) {
-    long long b = bitsOf(x);
-    int e = (int)((b >> 52) & 0x7FF);
-    if (e >= 2 && e <= 0x7FE) return fromBits(b - (1LL << 52));
+    const int hi = __double2hiint(x), lo = __double2loint(x), e = hi & 0x7FF00000;
+    if ((unsigned)e - 0x00200000u < 0x7FD00000u) return __hiloint2double(hi - 0x00100000, lo);
+    if (isZeroBits(x) || e == 0x7FF00000) return x;
     return halfNative(x);
 }
 __device__ __forceinline__ float halfOf(float x) { return x * .5f; }

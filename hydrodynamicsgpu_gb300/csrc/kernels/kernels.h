@@ -34,6 +34,7 @@ struct CombinePlan {
     int in;                   // slot of the stage input u^(k)
     int nops;
     CombineOp<real> ops[4];
+    int alphaAfter = -1;      // >= 0: the tableau whose zero-potential self-gravity pass the new state goes through
     real* slot[8];
 };
 
