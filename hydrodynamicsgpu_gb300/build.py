@@ -37,6 +37,7 @@ SOURCES = {
     "kernels/gravity.cu": ["--fmad=false"],
     "kernels/health.cu": ["--fmad=false"],
     "kernels/roe_fused.cu": ["--fmad=false"],
+    "kernels/roe_small.cu": ["--fmad=false"],
     "host/fits.cu": [],
     "host/adjoint.cu": [],
     "host/batch_solver.cu": [],

@@ -262,6 +262,21 @@ void ForwardEuler<real>::integrateFused(const std::function<void(real*, const Co
     throw ConfigError(HGPU_ERR_UNSUPPORTED, "fused stages need a Runge-Kutta integrator");
 }
 
+// state + deriv * dt as a Runge-Kutta row (beta dt of the one-stage tableau is dt): the
+// state plus the stage's deriv, into slot 1
+template <typename real>
+void ForwardEuler<real>::integrateSmall(const std::function<void(const CombinePlan<real>&)>& stageKernel, real* next) {
+    CombinePlan<real> plan{};
+    plan.nops = 1;
+    CombineOp<real>& op = plan.ops[0];
+    op.out = 1;
+    op.prior = 0;
+    op.hasBeta = 1;
+    plan.slot[0] = this->solver->state.template as<real>();
+    plan.slot[1] = next;
+    stageKernel(plan);
+}
+
 template <typename real>
 void ForwardEuler<real>::integrateZeroDeriv() {
     Solver<real>* s = this->solver;
@@ -409,6 +424,17 @@ template <typename real>
 void RungeKutta<real>::integrateFused(const std::function<void(real*, const CombinePlan<real>&)>& stageKernel) {
     for (int k = 0; k < order_; ++k) stageKernel(plans_[k].slot[inputSlot_[k]], plans_[k]);
     zeroDerivDone_ = false;
+}
+
+// plans_[k] never writes the slot stage k reads (buildStagePlans)
+template <typename real>
+void RungeKutta<real>::integrateSmall(const std::function<void(const CombinePlan<real>&)>& stageKernel, real*) {
+    for (int k = 0; k < order_; ++k) {
+        CombinePlan<real> plan = plans_[k];
+        plan.in = inputSlot_[k];
+        if (k == order_ - 1 && !alphaIsBinary_) plan.alphaAfter = tableau_;   // the self-gravity pass
+        stageKernel(plan);
+    }
 }
 
 template <typename real>
@@ -786,6 +812,10 @@ void Solver<real>::fixedDt() {
 template <typename real>
 void Solver<real>::update() {                                // Solver::update (Solver.cpp:521-546)
     this->launches_ = 0;
+    if (smallStep()) {
+        checkState();
+        return;
+    }
     boundary();
     initStep();
     if (rc.cfg.use_fixed_dt) fixedDt();
@@ -946,6 +976,49 @@ int Roe<real>::setFusedStages(bool on) {
     roeFusedPrepare();
     fused_ = true;
     return HGPU_OK;
+}
+
+// The grids that run as roe_small.cu's few launches: 1D, and 2D where the fused stage is
+// not offered (ForwardEuler or FP32: a 2D FP64 Runge-Kutta stage stays the four kernels that
+// hgpu_set_fused_stages replaces by two), up to the size where the recomputed faces cost
+// more than the launches.  us a step, this path / the kernels for large grids: 1D RK2
+// Superbee FP64 1028 cells 32.8 / 47.2, 65536 49 / 78, 262144 121 / 129, 2^20 446 / 434
+// (FP32 16 / 25, 20 / 29, 45 / 42, 143 / 106); 2D ForwardEuler FP64 64^2 35 / 66, 181^2
+// 66 / 69, 256^2 108 / 86; 2D RK2 FP32 64^2 19 / 35, 256^2 33 / 41, 362^2 48 / 49, 512^2
+// 76 / 61.
+template <typename real>
+bool Roe<real>::smallGrid() const {
+    const auto& c = this->rc.cfg;
+    const Grid& g = this->rc.grid;
+    if (g.dim > 2 || fused_ || c.compat != HGPU_COMPAT_REF || c.use_fixed_dt || this->livePotential()) return false;
+    for (int a = 0; a < g.dim; ++a)
+        if (g.S[a] < 6) return false;
+    if (g.dim == 2 && sizeof(real) == 8 && this->integrator->order() > 1) return false;
+    return g.V <= (g.dim == 1 ? 200000 : sizeof(real) == 4 ? 100000 : 32768);
+}
+
+template <typename real>
+bool Roe<real>::smallStep() {
+    if (!smallGrid()) return false;
+    const Grid& g = this->rc.grid;
+    real* state = this->state.template as<real>();
+    const bool fe = this->integrator->order() == 1;
+    real* next = fe ? this->flux.template as<real>() : state;      // the flux buffer is free: the fluxes stay on chip
+    this->launch("roe_prologue", 1, [&] {
+        launchSmallPrologue<real>(g, this->ph, this->methods, state, basis.template as<real>(), this->rc.cfg.integrator,
+                                  this->dtAcc.template as<CflAcc>(), this->sc(), this->stream);
+    });
+    this->integrator->integrateSmall([&](const CombinePlan<real>& plan) {
+        this->launch("roe_stage", 1, [&] {
+            launchSmallStage<real>(g, this->ph, this->rc.cfg.limiter, this->sc(), basis.template as<real>(), plan,
+                                   this->stream);
+        });
+    }, next);
+    if (fe)
+        this->launch("gravity_pass", 1, [&] {
+            launchSmallFinish<real>(g, this->methods, next, state, this->sc(), this->stream);
+        });
+    return true;
 }
 
 template <typename real>

@@ -124,6 +124,9 @@ public:
     // the self-gravity pass with a live potential: per callback the relaxation sweeps
     // (useGravity) and calcGravityDeriv of the stage state (SelfGravitation.cpp:100-124)
     virtual void integrateGravity() = 0;
+    // the stages by kernels that each form a stage's fluxes and apply its combine, for the
+    // small-grid step; ForwardEuler's writes to `next` instead of the state
+    virtual void integrateSmall(const std::function<void(const CombinePlan<real>& plan)>& stageKernel, real* next) = 0;
     virtual int order() const = 0;
     virtual int extraBuffers() const = 0;
     // true when the last stage's combine writes the new state and nothing after it in
@@ -142,6 +145,7 @@ public:
     using Integrator<real>::Integrator;
     void integrate(const std::function<void(real* stage)>& computeFlux) override;
     void integrateFused(const std::function<void(real* stage, const CombinePlan<real>& plan)>& stageKernel) override;
+    void integrateSmall(const std::function<void(const CombinePlan<real>& plan)>& stageKernel, real* next) override;
     void integrateZeroDeriv() override;
     void integrateGravity() override;
     int order() const override { return 1; }
@@ -154,6 +158,7 @@ public:
     RungeKutta(Solver<real>* s, int tableau);
     void integrate(const std::function<void(real* stage)>& computeFlux) override;
     void integrateFused(const std::function<void(real* stage, const CombinePlan<real>& plan)>& stageKernel) override;
+    void integrateSmall(const std::function<void(const CombinePlan<real>& plan)>& stageKernel, real* next) override;
     void integrateZeroDeriv() override;
     void integrateGravity() override;
     int order() const override { return order_; }
@@ -275,6 +280,9 @@ protected:
     virtual void initStep() {}
     virtual void calcTimestep() = 0;        // device-side; leaves dt and the step's constants in stepConst
     virtual void step() = 0;
+    // the whole of update() but the state check in few launches, for grids too small to fill
+    // the GPU; false: not for this grid and configuration
+    virtual bool smallStep() { return false; }
     void fixedDt();                         // the step's constants from the fixed dt
     void applyPotential();                  // SelfGravitation::applyPotential (SelfGravitation.cpp:100-124)
     bool potentialLive_ = false;            // useGravity, or a nonzero static potential was given
@@ -329,6 +337,8 @@ protected:
     struct alignas(64) TensorMap { unsigned char bytes[128]; };
     std::map<const void*, TensorMap> tensorMaps_;     // per stage buffer, for the fused y pass
     const void* tensorMapFor(const real* stage);
+    bool smallGrid() const;
+    bool smallStep() override;
     void fusedStage(real* stage, const CombinePlan<real>& plan);
     bool fusedActive() const override { return fused_; }
     void initBuffers() override;

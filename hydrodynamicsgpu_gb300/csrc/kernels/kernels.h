@@ -41,6 +41,20 @@ struct CombinePlan {
 // ---- boundary.cu ----
 template <typename real>
 void launchBoundary(const Grid& g, const int methods[3][2], real* state, cudaStream_t st);
+// ---- roe_small.cu: EulerRoe steps of small 1D and 2D grids (REF scheme, every axis of at
+// least 6 cells): ghost fill + eigenbasis + CFL timestep; one stage with its combine (the
+// stage input is plan.slot[plan.in]; no plan may write it); ForwardEuler's end ----
+struct CflAcc;
+template <typename real>
+void launchSmallPrologue(const Grid& g, const Phys<real>& ph, const int methods[3][2], real* state, real* basis,
+                         int integrator, CflAcc* acc, StepConst<real>* sc, cudaStream_t st);
+template <typename real>
+void launchSmallStage(const Grid& g, const Phys<real>& ph, int limiter, const StepConst<real>* sc, const real* basis,
+                      const CombinePlan<real>& plan, cudaStream_t st);
+template <typename real>
+void launchSmallFinish(const Grid& g, const int methods[3][2], const real* next, real* state, const StepConst<real>* sc,
+                       cudaStream_t st);
+
 int boundaryLaunches(const Grid& g);   // the kernels launchBoundary launches
 // the ghost fill along one axis over its transverse lines [t0, t1) (line t of axis a
 // addresses the cell with c[A] + S[A] * c[B] = t, A < B the other two axes)
