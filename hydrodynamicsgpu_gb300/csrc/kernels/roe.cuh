@@ -200,6 +200,47 @@ __device__ __forceinline__ void rightTransformDense(const real* rec, const real*
     }
 }
 
+// The rows of L x and R f (below) with a group's products.
+template <typename G, int D, int SIDE>
+__device__ __forceinline__ void leftRows(const double* rec, const double* x, double* y) {
+    typedef RoeRec<D> R_;
+    const int N = D + 2, E = N - 1;
+    double s0, s1, sE;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const int c = perm<SIDE>(j);
+        const double m = c == 0 ? rec[R_::LE0] : (c == 1 ? rec[R_::LE1] : rec[R_::L0 + c]);
+        const double p0 = G::mul(rec[R_::L0 + c], x[j]), p1 = G::mul(rec[R_::L1 + c], x[j]);
+        const double pE = c > 1 ? p0 : G::mul(m, x[j]);
+        s0 = j == 0 ? zfix(p0) : s0 + p0;
+        s1 = j == 0 ? zfix(p1) : s1 + p1;
+        sE = j == 0 ? zfix(pE) : sE + pE;
+    }
+    y[0] = s0;
+    y[1] = s1;
+    y[E] = sE;
+#pragma unroll
+    for (int t = 2; t < E; ++t) y[t] = zfix(G::mul(-rec[R_::VT + t - 2], x[0])) + x[perm<SIDE>(t)];
+}
+template <typename G, int D, int SIDE>
+__device__ __forceinline__ void rightRows(const double* rec, const double* f, double* F) {
+    typedef RoeRec<D> R_;
+    const int N = D + 2, E = N - 1;
+    double Fr[5];
+    Fr[0] = zfix(f[0]) + f[1] + f[E];
+    Fr[1] = zfix(G::mul(rec[R_::LAM0], f[0])) + G::mul(rec[R_::VX], f[1]) + G::mul(rec[R_::LAME], f[E]);
+    double s = zfix(G::mul(rec[R_::HM], f[0])) + G::mul(rec[R_::HV2], f[1]);
+#pragma unroll
+    for (int t = 2; t < E; ++t) {
+        const double vt = rec[R_::VT + t - 2];
+        Fr[t] = ((zfix(G::mul(vt, f[0])) + G::mul(vt, f[1])) + f[t]) + G::mul(vt, f[E]);
+        s = s + G::mul(vt, f[t]);
+    }
+    Fr[E] = s + G::mul(rec[R_::HP], f[E]);
+#pragma unroll
+    for (int g = 0; g < N; ++g) F[g] = Fr[perm<SIDE>(g)];
+}
+
 // y = L x with L in the global frame: y_i = sum_j L[i][perm(j)] x_j, j ascending.
 // FLAT: the caller's x is a difference of neighbouring states, often exactly zero.
 template <typename real, int D, int SIDE, bool FLAT = false>
@@ -223,6 +264,16 @@ __device__ __forceinline__ void leftTransform(const real* rec, const real* x, re
                 return;
             }
         }
+    }
+    if constexpr (sizeof(real) == 8) {
+        // the record's rows and x without a zero, with zeros, or neither (common.cuh's rule
+        // for finite operands then needs the dense sums)
+        if (warpAll(allInWindow<N>(x) & allInWindow<R_::NB - R_::VT>(rec + R_::VT)))
+            leftRows<GroupPlain, D, SIDE>(rec, x, y);
+        else if (warpAll(allInWindowOrZero<N>(x) & allInWindowOrZero<R_::NB - R_::VT>(rec + R_::VT)))
+            leftRows<GroupZeros, D, SIDE>(rec, x, y);
+        else leftTransformDense<real, D, SIDE>(rec, x, y);
+        return;
     }
     if (!allFinite<real, N>(x)) { leftTransformDense<real, D, SIDE>(rec, x, y); return; }
     // row 0 and row 1: dense
@@ -258,6 +309,13 @@ template <typename real, int D, int SIDE>
 __device__ __forceinline__ void rightTransform(const real* rec, const real* f, real* F) {
     typedef RoeRec<D> R_;
     const int N = D + 2, E = N - 1;
+    if constexpr (sizeof(real) == 8) {
+        if (warpAll(allInWindow<N>(f) & allInWindow<R_::L0>(rec))) rightRows<GroupPlain, D, SIDE>(rec, f, F);
+        else if (warpAll(allInWindowOrZero<N>(f) & allInWindowOrZero<R_::L0>(rec)))
+            rightRows<GroupZeros, D, SIDE>(rec, f, F);
+        else rightTransformDense<real, D, SIDE>(rec, f, F);
+        return;
+    }
     if (!allFinite<real, N>(f)) { rightTransformDense<real, D, SIDE>(rec, f, F); return; }
     real Fr[5];
     // row 0: [1, 1, 0.., 1]
@@ -352,36 +410,28 @@ __device__ __forceinline__ void roeFlux(const real* rec, const real* sL, const r
 // Each pass keeps far fewer values live than the fused form, so more warps fit per SM.
 // REC also stores the per-wave tape values of this pass (A, phi, phi', r; the caller
 // offsets tape to the face, as for roeFlux).
-// FLATQ: a wave whose Delta-q-tilde is +-0, with finite lambda and A, gets its
-// correction (lambda (+-0) / 2) A as the signed zero it is (sign(lambda) xor sign(dq)
-// xor sign(A)) on the bit patterns, skipping the product's and the halving's
-// out-of-line FP64 calls for zero operands.  Piecewise-constant states (the batched
-// four-quadrant problems) have such waves on most faces; the KH step measured it
-// slower, so it is the batched kernel's choice.
-template <int D, int SIDE, int LIM, bool REC = false, bool FLATQ = false>
-__device__ __forceinline__ void roeFluxCorrections(const double* rec, const double* dqL, const double* dq,
-                                                   const double* dqR, double dt_dx, int lim, double* corr,
-                                                   double* __restrict__ tape = nullptr, long long V = 0) {
-    typedef RoeRec<D> R_;
+struct GroupAny {
+    static __device__ __forceinline__ double mul(double x, double y) { return mulI(x, y); }
+    static __device__ __forceinline__ double div(double x, double y) { return divI(x, y); }
+    static __device__ __forceinline__ double half(double p) { return halfOf(p); }
+};
+template <typename G, int D, int SIDE, int LIM, bool REC>
+__device__ __forceinline__ void correctionsOf(const double* rec, const double* upwind, const double* dq, double dt_dx,
+                                              int lim, double* corr, double* __restrict__ tape, long long V) {
     const int N = D + 2;
-    const double vx = rec[R_::VX];
-    const bool midUp = geZero(vx);
-    const double midTheta = plusMinusOne(midUp);
-    const double midEpsTheta = mulI(vx, dt_dx) - midTheta;
+    const double vx = rec[RoeRec<D>::VX];
+    const double midTheta = plusMinusOne(geZero(vx));
+    const double midEpsTheta = G::mul(vx, dt_dx) - midTheta;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         const bool mid = i > 0 && i < N - 1;
         const double eigenvalue = roeEigenvalue<double, D>(rec, i);
-        const bool up = mid ? midUp : geZero(eigenvalue);
-        const double rTilde = divI(up ? dqL[i] : dqR[i], dq[i]);
-        const double theta = plusMinusOne(up);
+        const double theta = mid ? midTheta : plusMinusOne(geZero(eigenvalue));
+        const double rTilde = G::div(upwind[i], dq[i]);
         const double phi = slopeLimiter<double>(LIM >= 0 ? LIM : lim, rTilde);
-        const double epsMinusTheta = mid ? midEpsTheta : mulI(eigenvalue, dt_dx) - theta;
+        const double epsMinusTheta = mid ? midEpsTheta : G::mul(eigenvalue, dt_dx) - theta;
         const double A = theta + phi * epsMinusTheta;
-        if (FLATQ && isZeroBits(dq[i]) && finiteD(eigenvalue) && finiteD(A))
-            corr[i] = fromBits((bitsOf(eigenvalue) ^ bitsOf(dq[i]) ^ bitsOf(A)) & (long long)0x8000000000000000ULL);
-        else
-            corr[i] = halfOf(mulI(eigenvalue, dq[i])) * A;
+        corr[i] = G::half(G::mul(eigenvalue, dq[i])) * A;
         if (REC) {
             tape[((long long)FT_A * N + i) * V] = A;
             tape[((long long)FT_PHI * N + i) * V] = phi;
@@ -390,7 +440,31 @@ __device__ __forceinline__ void roeFluxCorrections(const double* rec, const doub
         }
     }
 }
+template <int D, int SIDE, int LIM, bool REC = false>
+__device__ __forceinline__ void roeFluxCorrections(const double* rec, const double* dqL, const double* dq,
+                                                   const double* dqR, double dt_dx, int lim, double* corr,
+                                                   double* __restrict__ tape = nullptr, long long V = 0) {
+    typedef RoeRec<D> R_;
+    const int N = D + 2;
+    const bool midUp = geZero(rec[R_::VX]);
+    double upwind[5];
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        upwind[i] = selectD(i > 0 && i < N - 1 ? midUp : geZero(roeEigenvalue<double, D>(rec, i)), dqL[i], dqR[i]);
+    const double lam[4] = {rec[R_::LAM0], rec[R_::VX], rec[R_::LAME], dt_dx};
+    if (warpAll(allInWindow<4>(lam) & allInWindow<N>(dq) & allInWindow<N>(upwind)))
+        correctionsOf<GroupPlain, D, SIDE, LIM, REC>(rec, upwind, dq, dt_dx, lim, corr, tape, V);
+    else if (warpAll(allInWindowOrZero<4>(lam) & allInWindowOrZero<N>(dq) & allInWindowOrZero<N>(upwind)))
+        correctionsOf<GroupZeros, D, SIDE, LIM, REC>(rec, upwind, dq, dt_dx, lim, corr, tape, V);
+    else correctionsOf<GroupAny, D, SIDE, LIM, REC>(rec, upwind, dq, dt_dx, lim, corr, tape, V);
+}
 
+// lambda (L avg) on the integer pipes where the warp's operands allow it: the transforms
+// pass is bound by the FP64 unit's sums (KH 2048^2: flux 785 -> 742 us a launch)
+static __device__ __noinline__ double lambdaNative(double a, double b) { return a * b; }
+__device__ __forceinline__ double lambdaProduct(double a, double b, bool plain) {
+    return plain ? GroupPlain::mul(a, b) : lambdaNative(a, b);
+}
 // REC also stores the tape values of this pass (L avg, and ft after the correction)
 template <int D, int SIDE, bool REC = false>
 __device__ __forceinline__ void roeFluxTransforms(const double* rec, const double* sL, const double* sR,
@@ -401,10 +475,12 @@ __device__ __forceinline__ void roeFluxTransforms(const double* rec, const doubl
 #pragma unroll
     for (int i = 0; i < N; ++i) avg[i] = halfOf(sR[i] + sL[i]);
     leftTransform<double, D, SIDE>(rec, avg, ft);
+    const double lam[3] = {rec[RoeRec<D>::LAM0], rec[RoeRec<D>::VX], rec[RoeRec<D>::LAME]};
+    const bool plain = warpAll(allInWindow<N>(ft) & allInWindow<3>(lam));
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         if (REC) tape[((long long)FT_Y * N + i) * V] = ft[i];
-        ft[i] = ft[i] * roeEigenvalue<double, D>(rec, i) - corr[i];
+        ft[i] = lambdaProduct(ft[i], roeEigenvalue<double, D>(rec, i), plain) - corr[i];
         if (REC) tape[((long long)FT_F * N + i) * V] = ft[i];
     }
     rightTransform<double, D, SIDE>(rec, ft, F);
