@@ -71,6 +71,7 @@ __device__ __forceinline__ bool fmaxTakesFirst(double x, double y) {
 __device__ __forceinline__ double selectD(bool c, double a, double b) {
     return fromBits(c ? bitsOf(a) : bitsOf(b));
 }
+__device__ __forceinline__ float selectD(bool c, float a, float b) { return c ? a : b; }
 __device__ __forceinline__ double fminLibm(double x, double y) { return selectD(fminTakesFirst(x, y), x, y); }
 __device__ __forceinline__ double fmaxLibm(double x, double y) { return selectD(fmaxTakesFirst(x, y), x, y); }
 // c ? 1. : -1., selected as an integer
@@ -221,6 +222,44 @@ __device__ __forceinline__ double divI(double x, double y) {
 }
 __device__ __forceinline__ float divI(float x, float y) { return x / y; }
 
+// sqrt(x) on the integer pipes, bit-identical to the FP64 unit's: x normal and positive (its
+// words given).  With M in [1, 4) the significand, doubled where the exponent is odd, and
+// a = M / 4: y ~ 1 / sqrt(a) is seeded by the FP32 reciprocal square root of a's top bits
+// (rounded up, the result lowered by 4 units), refined by two fixed-point Newton steps
+// y += y (1 - a y^2) / 2 that keep it from below (2^-28, then 2^-57); q = floor(2^53 a y) is
+// the truncated root or one less, and the remainder, exact modulo 2^64, against q rounds it
+// to nearest (a root is never a tie).  Some 60 instructions against about ten FP64
+// operations of 64 issue slots each: KH 2048^2 eigenbasis 867 -> 525 us a launch (with roe.cuh's left rows off the FP64 unit too), HLLC wave
+// speeds at 1021x1030 154 -> 105 us, at 160x144x136 889 -> 713 us.
+__device__ __forceinline__ double rootBits(unsigned xh, unsigned xl) {
+    const unsigned odd = (~xh >> 20) & 1u, mh = (xh & 0xFFFFFu) | 0x100000u;
+    const unsigned ah = __funnelshift_l(xl, mh, 10 + odd), al = xl << (10 + odd);          // a 2^64
+    float rf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;"
+        : "=f"(rf)
+        : "f"(__uint_as_float(((0x3E800000u + (odd << 23)) | (__funnelshift_l(xl, mh, 3) & 0x7FFFFFu)) + 1u)));
+    const unsigned y0 = (__float_as_uint(rf) - 4u) << 8;                                   // y 2^31
+    const unsigned e0 = (unsigned)((0x4000000000000000ull - (unsigned long long)ah * __umulhi(y0, y0)) >> 12);
+    const unsigned y1 = y0 + (__umulhi(y0, e0) >> 19) - 4u;
+    const unsigned long long a = ((unsigned long long)ah << 32) | al;
+    const unsigned long long e1 = 0x3FFFFFFFFFFFFFFFull - __umul64hi(a, (unsigned long long)y1 * y1);   // < 2^35
+    const unsigned long long y2 = ((unsigned long long)y1 << 32) + (((unsigned long long)y1 * (unsigned)(e1 >> 4)) >> 27);
+    const unsigned long long q = __umul64hi(a, y2) >> 10;
+    const unsigned q0 = (unsigned)q, q1 = (unsigned)(q >> 32);
+    const unsigned long long lo = (unsigned long long)q0 * q0;
+    const unsigned long long rem = ((unsigned long long)((xl << (20 + odd)) - ((unsigned)(lo >> 32) + 2u * q0 * q1)) << 32) -
+                                   (unsigned)lo;
+    const unsigned top = ((((xh >> 20) + 1023u) >> 1) - 1u) << 20;
+    return __longlong_as_double((long long)(((unsigned long long)top << 32) + q + (rem > q ? 1u : 0u)));
+}
+static __device__ __noinline__ double sqrtNative(double x) { return sqrt(x); }
+__device__ __forceinline__ double sqrtI(double x) {
+    const unsigned h = (unsigned)__double2hiint(x);
+    if (h - 0x00100000u >= 0x7FE00000u) return sqrtNative(x);     // negative, zero, subnormal, Inf, NaN
+    return rootBits(h, (unsigned)__double2loint(x));
+}
+__device__ __forceinline__ float sqrtI(float x) { return sqrt(x); }
+
 // Arithmetic on a group of operands that were tested once, without a branch of its own, so
 // that the compiler can interleave the independent products and quotients (each a dependent
 // chain of some 30 integer instructions, which a warp otherwise waits out one by one).
@@ -315,6 +354,58 @@ __device__ __forceinline__ double quotBy(double x, const Divisor<double>& d) {
     }
     return quotientBits(xh, xl, yh, yl, d.v);
 }
+
+// x / d for x and d.b in the window (GroupPlain's quotient by a shared divisor)
+__device__ __forceinline__ double quotPlain(double x, const Divisor<double>& d) {
+    return quotientBits((unsigned)__double2hiint(x), (unsigned)__double2loint(x), (unsigned)__double2hiint(d.b),
+                        (unsigned)__double2loint(d.b), d.v);
+}
+
+// The operations of a longer computation: AnyOps tests each operand pair (mulI, divI);
+// CheckedOps assumes ordinary magnitudes and keeps in `ok` whether every operand had one, for
+// the caller to do the whole computation again with AnyOps if not.
+template <typename real>
+struct AnyOps {
+    bool ok = true;
+    __device__ __forceinline__ real mul(real x, real y) { return mulI(x, y); }
+    __device__ __forceinline__ real div(real x, real y) { return divI(x, y); }
+    __device__ __forceinline__ real half(real x) { return halfOf(x); }
+    __device__ __forceinline__ real root(real x) { return sqrtI(x); }
+    __device__ __forceinline__ Divisor<real> divisor(real b) { return divisorOf(b); }
+    __device__ __forceinline__ real quot(real x, const Divisor<real>& d) { return quotBy(x, d); }
+};
+struct CheckedOps {
+    bool ok = true;
+    __device__ __forceinline__ double mul(double x, double y) {
+        ok &= inWindow(x) & inWindow(y);
+        return GroupPlain::mul(x, y);
+    }
+    __device__ __forceinline__ double div(double x, double y) {
+        ok &= inWindow(x) & inWindow(y);
+        return GroupPlain::div(x, y);
+    }
+    __device__ __forceinline__ double half(double x) {
+        ok &= inWindow(x);
+        return GroupPlain::half(x);
+    }
+    __device__ __forceinline__ double root(double x) {
+        ok &= inWindow(x) & (__double2hiint(x) >= 0);
+        return rootBits((unsigned)__double2hiint(x), (unsigned)__double2loint(x));
+    }
+    // 2 x of a product (exact)
+    __device__ __forceinline__ double twice(double x) {
+        ok &= inWindow(x);
+        return __hiloint2double(__double2hiint(x) + 0x00100000, __double2loint(x));
+    }
+    __device__ __forceinline__ Divisor<double> divisor(double b) {
+        ok &= inWindow(b);
+        return {b, recipBits((unsigned)__double2hiint(b), (unsigned)__double2loint(b))};
+    }
+    __device__ __forceinline__ double quot(double x, const Divisor<double>& d) {
+        ok &= inWindow(x);
+        return quotPlain(x, d);
+    }
+};
 
 // (float)((double)c - (double)a * (double)b) for floats, on the FP32 pipes.  The product
 // is exact in double (48 bits), so the value is c - a*b rounded to 53 bits and then to 24;

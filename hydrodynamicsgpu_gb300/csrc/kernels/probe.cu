@@ -50,6 +50,8 @@ __global__ void selftestKernel(unsigned long long seed, long long cases, unsigne
         const double pm = x * y, qm = mulI(x, y), pd = x / y, qd = divI(x, y);
         if (bitsOf(pm) != bitsOf(qm) && !(pm != pm && qm != qm)) ++nm;
         if (bitsOf(pd) != bitsOf(qd) && !(pd != pd && qd != qd)) ++nd;
+        const double ps = sqrt(x), qs = sqrtI(x);
+        if (bitsOf(ps) != bitsOf(qs) && !(ps != ps && qs != qs)) ++nd;
     }
     if (nm) atomicAdd(&bad[0], nm);
     if (nd) atomicAdd(&bad[1], nd);
@@ -91,7 +93,7 @@ int selftestLimiters(unsigned long long seed, long long cases, long long* bad) {
     return 0;
 }
 
-// mismatches of mulI / divI against the FP64 unit over `cases` seeded operand pairs
+// mismatches of mulI, and of divI and sqrtI together, against the FP64 unit over `cases` seeded operand pairs
 int selftestFp64Ops(unsigned long long seed, long long cases, long long* mulBad, long long* divBad) {
     unsigned long long* bad = nullptr;
     if (cudaMalloc(&bad, 2 * sizeof(unsigned long long)) != cudaSuccess) return -1;

@@ -11,6 +11,8 @@
 // bit-identical; sums over matrix columns keep the reference's column order in the
 // global frame (see common.cuh for the zero/unit-coefficient rule).
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "fp64ops.cuh"
 #include "limiter_dual.cuh"
@@ -18,12 +20,8 @@
 namespace hgpu {
 
 // A product on the FP64 unit, never contracted into an fma (so the same in translation
-// units built with and without --fmad=false).  The eigenbasis kernel issues far more
-// integer than FP64 instructions (its quotients and the record's products on the
-// integer pipes, the FP64 unit at ~59 %): its per-cell products and the left rows'
-// products run here instead of through mulI, which balanced the pipes (KH 2048^2 step
-// 7.703 -> 7.688 ms, the 512-problem batched sweep 24.42 -> 24.17 ms; every product
-// through mulN was slower, 7.82 ms).
+// units built with and without --fmad=false): the eigenbasis kernel's per-cell products,
+// and the left rows' where the face's operands are not all ordinary numbers.
 __device__ __forceinline__ double mulN(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mulN(float a, float b) { return __fmul_rn(a, b); }
 
@@ -69,11 +67,24 @@ __device__ __forceinline__ void roePrim(const real* s, real gamma, RoePrim<real,
     const int E = D + 1;
     const real gm1 = gamma - (real)1.f;
     real rho = s[0];
-    const Divisor<real> byRho = divisorOf(rho);
-    real invDensity = quotBy((real)1.f, byRho);                          // `1.f / density`
+    real invDensity;                                                     // `1.f / density`
     // VELOCITY(ptr) = (m..., 0)/rho componentwise (res/include/HydroGPU/Euler.h:6-12)
+    bool done = false;
+    if constexpr (sizeof(real) == 8) {
+        if (warpAll(inWindow(rho) & allInWindow<D>(s + 1))) {
+            const Divisor<real> byRho = {rho, recipBits((unsigned)__double2hiint(rho), (unsigned)__double2loint(rho))};
+            invDensity = quotPlain(1., byRho);
 #pragma unroll
-    for (int k = 0; k < D; ++k) P.v[k] = quotBy(s[1 + k], byRho);
+            for (int k = 0; k < D; ++k) P.v[k] = quotPlain(s[1 + k], byRho);
+            done = true;
+        }
+    }
+    if (!done) {
+        const Divisor<real> byRho = divisorOf(rho);
+        invDensity = quotBy((real)1.f, byRho);
+#pragma unroll
+        for (int k = 0; k < D; ++k) P.v[k] = quotBy(s[1 + k], byRho);
+    }
     // dot(v,v) over 4 components; the zero components add +0 to a non-negative sum
     real vv = mulN(P.v[0], P.v[0]);
 #pragma unroll
@@ -85,45 +96,66 @@ __device__ __forceinline__ void roePrim(const real* s, real gamma, RoePrim<real,
     P.phi = phi;
     real pressure = mulN(mulN(gm1, rho), energyInternal);
     P.h = energyTotal + mulN(pressure, invDensity);
-    P.w = sqrt(rho);
+    P.w = sqrtI(rho);
 }
 
 // Per-face part (res/EulerRoe.cl:85-226): Roe averages, eigenvalues, R and L.
-template <typename real, int D, int SIDE, bool GRAV = false>
-__device__ __forceinline__ void roeBasisFromPrim(const RoePrim<real, D>& L, const RoePrim<real, D>& R, real gamma,
-                                                 real* rec) {
+template <typename O, typename real, int D, int SIDE, bool GRAV>
+__device__ __forceinline__ void roeBasisOf(O& o, const RoePrim<real, D>& L, const RoePrim<real, D>& R, real gamma,
+                                           real* rec) {
     typedef RoeRec<D> R_;
     const int E = D + 1;
     const real gm1 = gamma - (real)1.f;
-    real norm = divI((real)1.f, L.w + R.w);
+    real norm = o.div((real)1.f, L.w + R.w);
     real v[3];
 #pragma unroll
-    for (int k = 0; k < D; ++k) v[k] = mulI(mulI(L.w, L.v[k]) + mulI(R.w, R.v[k]), norm);
-    real enthalpyTotal = mulI(mulI(L.w, L.h) + mulI(R.w, R.h), norm);
-    real velocitySq = mulI(v[0], v[0]);
+    for (int k = 0; k < D; ++k) v[k] = o.mul(o.mul(L.w, L.v[k]) + o.mul(R.w, R.v[k]), norm);
+    real enthalpyTotal = o.mul(o.mul(L.w, L.h) + o.mul(R.w, R.h), norm);
+    real velocitySq = o.mul(v[0], v[0]);
 #pragma unroll
-    for (int k = 1; k < D; ++k) velocitySq = velocitySq + mulI(v[k], v[k]);
-    real hc = enthalpyTotal - halfOf(velocitySq);
+    for (int k = 1; k < D; ++k) velocitySq = velocitySq + o.mul(v[k], v[k]);
+    const real halfVelocitySq = o.half(velocitySq);
+    real hc = enthalpyTotal - halfVelocitySq;
     if (GRAV) {                                                          // - energyPotential (Roe average)
-        const real energyPotential = mulI(mulI(L.w, L.phi) + mulI(R.w, R.phi), norm);
+        const real energyPotential = o.mul(o.mul(L.w, L.phi) + o.mul(R.w, R.phi), norm);
         hc = hc - energyPotential;
     }
-    real c = sqrt(mulI(hc, gm1));
+    real c = o.root(o.mul(hc, gm1));
     // rotate: normal velocity first (res/EulerRoe.cl:101-110)
     real vx = v[SIDE];
     real vt[2] = {0, 0};
     if (D > 1) vt[0] = (SIDE == 1) ? v[0] : v[1];
     if (D > 2) vt[1] = (SIDE == 2) ? v[0] : v[2];
-    real cvx = mulI(c, vx);
+    real cvx = o.mul(c, vx);
     rec[R_::LAM0] = vx - c;
     rec[R_::VX] = vx;
     rec[R_::LAME] = vx + c;
     rec[R_::HM] = enthalpyTotal - cvx;
-    rec[R_::HV2] = halfOf(velocitySq);
+    rec[R_::HV2] = halfVelocitySq;
 #pragma unroll
     for (int t = 0; t < D - 1; ++t) rec[R_::VT + t] = vt[t];
     rec[R_::HP] = enthalpyTotal + cvx;
-    real invDenom = divI((real).5f, mulI(c, c));
+    real invDenom = o.div((real).5f, o.mul(c, c));
+    if constexpr (std::is_same<O, CheckedOps>::value) {
+        // the same entries for ordinary magnitudes, where scaling by 2 is exact: row 1 is
+        // twice row 0's products
+        const real hv = o.mul(o.half(gm1), velocitySq), gvx = o.mul(gm1, vx), gi = o.mul(gm1, invDenom);
+        rec[R_::L0 + 0] = o.mul(hv + cvx, invDenom);
+        rec[R_::L0 + 1] = o.mul(-(c + gvx), invDenom);
+        rec[R_::L0 + E] = gi;
+        rec[R_::L1 + 0] = (real)1.f - o.mul(o.mul(gm1, velocitySq), invDenom);
+        rec[R_::L1 + 1] = o.twice(o.mul(gvx, invDenom));
+        rec[R_::L1 + E] = -o.twice(gi);
+#pragma unroll
+        for (int t = 0; t < D - 1; ++t) {
+            const real g = o.mul(o.mul(gm1, vt[t]), invDenom);
+            rec[R_::L0 + 2 + t] = -g;
+            rec[R_::L1 + 2 + t] = o.twice(g);
+        }
+        rec[R_::LE0] = o.mul(hv - cvx, invDenom);
+        rec[R_::LE1] = o.mul(c - gvx, invDenom);
+        return;
+    }
     real hv = mulN(mulN((real).5f, gm1), velocitySq);                    // .5f * (gamma - 1.f) * velocitySq
     real gvx = mulN(gm1, vx);
     rec[R_::L0 + 0] = mulN(hv + cvx, invDenom);
@@ -138,6 +170,22 @@ __device__ __forceinline__ void roeBasisFromPrim(const RoePrim<real, D>& L, cons
     rec[R_::L1 + E] = mulN(mulN(-gm1, (real)2.f), invDenom);
     rec[R_::LE0] = mulN(hv - cvx, invDenom);
     rec[R_::LE1] = mulN(c - gvx, invDenom);
+}
+
+// by CheckedOps where the warp's velocities are ordinary numbers (not exact zeros), by AnyOps
+// otherwise or if an operand on the way was not one
+template <typename real, int D, int SIDE, bool GRAV = false>
+__device__ __forceinline__ void roeBasisFromPrim(const RoePrim<real, D>& L, const RoePrim<real, D>& R, real gamma,
+                                                 real* rec) {
+    if constexpr (sizeof(real) == 8) {
+        if (warpAll(allInWindow<D>(L.v) & allInWindow<D>(R.v))) {
+            CheckedOps o;
+            roeBasisOf<CheckedOps, real, D, SIDE, GRAV>(o, L, R, gamma, rec);
+            if (warpAll(o.ok)) return;
+        }
+    }
+    AnyOps<real> o;
+    roeBasisOf<AnyOps<real>, real, D, SIDE, GRAV>(o, L, R, gamma, rec);
 }
 
 // Eigen basis of one interface from the two cell states.
