@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kThreads) ghostKernel(Grid g, int N, Methods b
 // the last stage (as a pass of its own over the state: 3D 160x144x136 RungeKutta2TVD 482 us
 // of the step, 3D 99x90x86 RungeKutta3TVD 211 us; folded, 60 and 55 us more of combine)
 template <typename real, int D, bool POST>
-__global__ void __launch_bounds__(kThreads, 5) derivCombineKernel(Grid g, Phys<real> ph, const real* __restrict__ flux,
+__global__ void __launch_bounds__(kThreads, D < 3 || sizeof(real) == 4 ? 5 : 4) derivCombineKernel(Grid g, Phys<real> ph, const real* __restrict__ flux,
                                                                CombinePlan<real> plan,
                                                                const StepConst<real>* __restrict__ sc, long long c0,
                                                                long long c1) {
