@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kThreads) hllcWaveTileKernel(Grid g, Phys<real
     dependentLaunch();
     typedef FluxTile<D> T;
     constexpr int HX = T::X + 1, HY = T::Y + 1, HZ = D > 2 ? T::Z + 1 : 1;
-    __shared__ Prim<real, D> prim[HX * HY * HZ];
+    __shared__ WavePrim<real, D> prim[HX * HY * HZ];
     const int x0 = blockIdx.x * T::X;
     const int y0 = D == 2 ? s0 + (int)blockIdx.y * T::Y : (int)blockIdx.y * T::Y;
     const int z0 = D == 2 ? 0 : s0 + (int)blockIdx.z * T::Z;

@@ -1,6 +1,8 @@
 // hllc_cells.cuh -- per-cell bodies of the EulerHLLC kernels (res/EulerHLLC.cl),
 // shared by the single-problem kernels (hllc.cu) and the batched kernels (batch.cu).
 #pragma once
+#include <type_traits>
+
 #include "kernels.h"
 
 namespace hgpu {
@@ -16,6 +18,12 @@ __device__ __forceinline__ void loadRotated(const real* __restrict__ s, long lon
 template <typename real, int D>
 struct Prim {
     real density, invDensity, v[3], velocitySq, energyTotal, pressure, enthalpyTotal, potential;
+};
+// with the square roots that the wave speeds of all the cell's faces share: the sound speed
+// and, for EulerHLL, the Roe weight sqrt(density)
+template <typename real, int D>
+struct WavePrim : Prim<real, D> {
+    real c, w;
 };
 
 // the part of primitives() that follows the velocities: |v|^2 (components in order),
@@ -40,10 +48,24 @@ template <typename real, int D, bool GRAV = false>
 __device__ __forceinline__ void primitives(const real* st, real gamma, Prim<real, D>& p, real phi = (real)0) {
     const int E = D + 1;
     p.density = st[0];
-    const Divisor<real> byRho = divisorOf(p.density);
-    p.invDensity = quotBy((real)1, byRho);   // FP32: the double quotient rounded to float is the float quotient
+    // (FP32: the double quotient rounded to float is the float quotient)
+    bool done = false;
+    if constexpr (sizeof(real) == 8) {
+        if (warpAll(inWindow(p.density) & allInWindow<D>(st + 1))) {
+            const Divisor<real> byRho = {p.density, recipBits((unsigned)__double2hiint(p.density),
+                                                              (unsigned)__double2loint(p.density))};
+            p.invDensity = quotPlain(1., byRho);
 #pragma unroll
-    for (int k = 0; k < D; ++k) p.v[k] = quotBy(st[1 + k], byRho);
+            for (int k = 0; k < D; ++k) p.v[k] = quotPlain(st[1 + k], byRho);
+            done = true;
+        }
+    }
+    if (!done) {
+        const Divisor<real> byRho = divisorOf(p.density);
+        p.invDensity = quotBy((real)1, byRho);
+#pragma unroll
+        for (int k = 0; k < D; ++k) p.v[k] = quotBy(st[1 + k], byRho);
+    }
     p.energyTotal = mulI(st[E], p.invDensity);
     p.potential = phi;
     primitivesFromVelocity<real, D, GRAV>(gamma, p);
@@ -65,13 +87,16 @@ __device__ __forceinline__ void rotatePrim(const Prim<real, D>& p, real gamma, P
 }
 
 // sl, sr of one face (EulerHLLC.cl:85-97)
+template <bool HLL, typename real, int D>
+__device__ __forceinline__ real soundSpeed(double gm1, const Prim<real, D>& P);
 template <typename real, int D, int SIDE>
-__device__ __forceinline__ void waveFaceFromPrim(const Grid& g, const Phys<real>& ph, double gq,
-                                                 const Prim<real, D>& L, const Prim<real, D>& R,
-                                                 real* __restrict__ waves, long long c);
+__device__ __forceinline__ void waveFaceFromPrim(const Grid& g, double gq, const Prim<real, D>& L,
+                                                 const Prim<real, D>& R, real cL, real cR, real* __restrict__ waves,
+                                                 long long c);
 template <typename real, int D, int SIDE, bool GRAV>
 __device__ __forceinline__ void hllWaveFaceFromPrim(const Grid& g, const Phys<real>& ph, const Prim<real, D>& L,
-                                                    const Prim<real, D>& R, real* __restrict__ waves, long long c);
+                                                    const Prim<real, D>& R, real cL, real cR, real wL, real wR,
+                                                    real* __restrict__ waves, long long c);
 
 template <typename real, int D, int SIDE, bool GRAV = false>
 __device__ __forceinline__ void waveFace(const Grid& g, const Phys<real>& ph, double gq, const real* __restrict__ state,
@@ -84,26 +109,33 @@ __device__ __forceinline__ void waveFace(const Grid& g, const Phys<real>& ph, do
     Prim<real, D> L, R;
     primitives<real, D, GRAV>(sL, ph.gamma, L, GRAV ? pot[c - g.step[SIDE]] : (real)0);
     primitives<real, D, GRAV>(sR, ph.gamma, R, GRAV ? pot[c] : (real)0);
-    waveFaceFromPrim<real, D, SIDE>(g, ph, gq, L, R, waves, c);
+    const double gm1 = (double)ph.gamma - 1.;
+    waveFaceFromPrim<real, D, SIDE>(g, gq, L, R, soundSpeed<false>(gm1, L), soundSpeed<false>(gm1, R), waves, c);
 }
 
-// the rest of waveFace, given the face's two cells' primitives (rotated to the face)
+// sound speed of a cell in the face's frame (EulerHLLC.cl:85-86, EulerHLL.cl:64-75; `.5 *`
+// is a double literal in the latter, which FP32 promotes)
+template <bool HLL, typename real, int D>
+__device__ __forceinline__ real soundSpeed(double gm1, const Prim<real, D>& P) {
+    if (HLL) return (real)sqrtI(mulI(gm1, (double)P.enthalpyTotal - halfOf((double)P.velocitySq)));
+    return (real)sqrtI(mulI(gm1, (double)(P.enthalpyTotal - halfOf(P.velocitySq))));
+}
+
+// the rest of waveFace, given the face's two cells' primitives (rotated to the face) and
+// sound speeds
 template <typename real, int D, int SIDE>
-__device__ __forceinline__ void waveFaceFromPrim(const Grid& g, const Phys<real>& ph, double gq,
-                                                 const Prim<real, D>& L, const Prim<real, D>& R,
-                                                 real* __restrict__ waves, long long c) {
-    const double gm1 = (double)ph.gamma - 1.;
-    real cL = (real)sqrt(mulI(gm1, (double)(L.enthalpyTotal - halfOf(L.velocitySq))));
-    real cR = (real)sqrt(mulI(gm1, (double)(R.enthalpyTotal - halfOf(R.velocitySq))));
+__device__ __forceinline__ void waveFaceFromPrim(const Grid& g, double gq, const Prim<real, D>& L,
+                                                 const Prim<real, D>& R, real cL, real cR, real* __restrict__ waves,
+                                                 long long c) {
     // .5f * (pL + pR) - .5f * (vR - vL) * .5f * (rhoL + rhoR) * .5f * (cL + cR), halvings exact
     real pressureStar = (real)fmaxLibm(0., (double)(halfOf(L.pressure + R.pressure) -
                                                     mulI(halfOf(mulI(halfOf(halfOf(R.v[0] - L.v[0])),
                                                                      L.density + R.density)),
                                                          cL + cR)));
     real qL = leD(pressureStar, L.pressure) ? (real)1.
-                                         : (real)sqrt(1. + mulI(gq, (double)divI(pressureStar, L.pressure) - 1.));
+                                         : (real)sqrtI(1. + mulI(gq, (double)divI(pressureStar, L.pressure) - 1.));
     real qR = leD(pressureStar, R.pressure) ? (real)1.
-                                         : (real)sqrt(1. + mulI(gq, (double)divI(pressureStar, R.pressure) - 1.));
+                                         : (real)sqrtI(1. + mulI(gq, (double)divI(pressureStar, R.pressure) - 1.));
     waves[((long long)SIDE * 2 + 0) * g.V + c] = L.v[0] - mulI(cL, qL);
     waves[((long long)SIDE * 2 + 1) * g.V + c] = R.v[0] + mulI(cR, qR);
 }
@@ -122,17 +154,17 @@ __device__ __forceinline__ void hllWaveFace(const Grid& g, const Phys<real>& ph,
     Prim<real, D> L, R;
     primitives<real, D, GRAV>(sL, ph.gamma, L, GRAV ? pot[c - g.step[SIDE]] : (real)0);
     primitives<real, D, GRAV>(sR, ph.gamma, R, GRAV ? pot[c] : (real)0);
-    hllWaveFaceFromPrim<real, D, SIDE, GRAV>(g, ph, L, R, waves, c);
+    const double gm1 = (double)ph.gamma - 1.;
+    hllWaveFaceFromPrim<real, D, SIDE, GRAV>(g, ph, L, R, soundSpeed<true>(gm1, L), soundSpeed<true>(gm1, R),
+                                             sqrtI(L.density), sqrtI(R.density), waves, c);
 }
 
 // the rest of hllWaveFace, given the face's two cells' primitives (rotated to the face)
 template <typename real, int D, int SIDE, bool GRAV>
 __device__ __forceinline__ void hllWaveFaceFromPrim(const Grid& g, const Phys<real>& ph, const Prim<real, D>& L,
-                                                    const Prim<real, D>& R, real* __restrict__ waves, long long c) {
+                                                    const Prim<real, D>& R, real cL, real cR, real wL, real wR,
+                                                    real* __restrict__ waves, long long c) {
     const double gm1 = (double)ph.gamma - 1.;
-    const real cL = (real)sqrt(mulI(gm1, (double)L.enthalpyTotal - halfOf((double)L.velocitySq)));
-    const real cR = (real)sqrt(mulI(gm1, (double)R.enthalpyTotal - halfOf((double)R.velocitySq)));
-    const real wL = sqrt(L.density), wR = sqrt(R.density);
     const real norm = (real)divI(1., (double)(wL + wR));
     real v[3], vv;
 #pragma unroll
@@ -144,7 +176,7 @@ __device__ __forceinline__ void hllWaveFaceFromPrim(const Grid& g, const Phys<re
     // - energyPotential, the Roe average of the potential (zero without GRAV: left out)
     double hc = (double)H - halfOf((double)vv);
     if (GRAV) hc = hc - (double)mulI(mulI(wL, L.potential) + mulI(wR, R.potential), norm);
-    const real cs = (real)sqrt(mulI(gm1, hc));
+    const real cs = (real)sqrtI(mulI(gm1, hc));
     waves[((long long)SIDE * 2 + 0) * g.V + c] = fminLibm(L.v[0] - cL, v[0] - cs);
     waves[((long long)SIDE * 2 + 1) * g.V + c] = fmaxLibm(R.v[0] + cR, v[0] + cs);
 }
@@ -221,60 +253,96 @@ __device__ __forceinline__ bool hllcFace(const Grid& g, const Phys<real>& ph, co
     return hllcFaceFromPrim<real, D, SIDE>(g, stL, stR, L, R, waves, fluxBuf, c);
 }
 
+// physical flux of one side along the face's normal, its mass flux given
+template <typename O, typename real, int D>
+__device__ __forceinline__ void sideFlux(O& o, const Prim<real, D>& P, real mass, real* f) {
+    f[0] = mass;
+    f[1] = o.mul(mass, P.v[0]) + P.pressure;
+#pragma unroll
+    for (int k = 1; k < D; ++k) f[1 + k] = o.mul(o.mul(P.density, P.v[k]), P.v[0]);
+    f[D + 1] = o.mul(o.mul(P.density, P.enthalpyTotal), P.v[0]);
+}
+
+// The HLLC flux of one face (rotated frame) into `flux`; returns 0 where no branch applies.
+// The reference forms both sides' physical fluxes and then picks a branch; each branch uses
+// one side's, so the side is chosen first (by sl, sStar and sr) and its state, primitives and
+// wave speed selected: every value formed is the reference's.  With the products and quotients
+// by CheckedOps: flux 316 -> 182 us a launch at 1021x1030, 2300 -> 1465 us at 160x144x136.
+template <typename O, typename real, int D>
+__device__ __forceinline__ bool hllcFluxOf(O& o, const real* stL, const real* stR, const Prim<real, D>& L,
+                                           const Prim<real, D>& R, real sl, real sr, real* flux) {
+    const int N = D + 2, E = N - 1;
+    const real massL = o.mul(L.density, L.v[0]), massR = o.mul(R.density, R.v[0]);
+    const real dL = sl - L.v[0], dR = sr - R.v[0];
+    const real rL = o.mul(L.density, dL), rR = o.mul(R.density, dR);
+    const real sStar = o.div(o.mul(massR, dR) - o.mul(massL, dL) + L.pressure - R.pressure, rR - rL);
+    // (the branch tests on the bit patterns: double compares issue to the FP64 unit)
+    const bool allLeft = geZero(sl);
+    const bool left = allLeft || (leZero(sl) && geZero(sStar));
+    const bool rightStar = leZero(sStar) && geZero(sr);
+    const bool taken = left || rightStar || leZero(sr);
+    const bool star = left ? !allLeft : rightStar;
+    Prim<real, D> P;
+    P.density = selectD(left, L.density, R.density);
+    P.pressure = selectD(left, L.pressure, R.pressure);
+    P.enthalpyTotal = selectD(left, L.enthalpyTotal, R.enthalpyTotal);
+#pragma unroll
+    for (int k = 0; k < D; ++k) P.v[k] = selectD(left, L.v[k], R.v[k]);
+    sideFlux(o, P, selectD(left, massL, massR), flux);
+    if (star) {
+        const real pressureLR = o.half(L.pressure + R.pressure + o.mul(rL, sStar - L.v[0]) + o.mul(rR, sStar - R.v[0]));
+        const real s = selectD(left, sl, sr), sp = o.mul(s, pressureLR);
+        const Divisor<real> den = o.divisor(s - sStar);          // every component divides by it
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            real t = o.mul(sStar, o.mul(s, selectD(left, stL[j], stR[j])) - flux[j]);
+            if (j == 1) t = t + sp;
+            if (j == E) t = t + o.mul(sp, sStar);
+            flux[j] = o.quot(t, den);
+        }
+    }
+    return taken;
+}
+
+// whether the operands that the fluxes start from are all of an ordinary magnitude in every
+// lane of the warp (gas at rest is not: its lanes go straight to AnyOps)
+template <int D>
+__device__ __forceinline__ bool ordinaryFace(const double* stL, const double* stR, const Prim<double, D>& L,
+                                             const Prim<double, D>& R, double sl, double sr) {
+    return warpAll(allInWindow<D + 2>(stL) & allInWindow<D + 2>(stR) & allInWindow<D>(L.v) & allInWindow<D>(R.v) &
+                   inWindow(sl) & inWindow(sr));
+}
+template <int D>
+__device__ __forceinline__ bool ordinaryFace(const float*, const float*, const Prim<float, D>&, const Prim<float, D>&,
+                                             float, float) {
+    return false;
+}
+
 // the rest of hllcFace, given the face's rotated states and their primitives
 template <typename real, int D, int SIDE>
 __device__ __forceinline__ bool hllcFaceFromPrim(const Grid& g, const real* stL, const real* stR,
                                                  const Prim<real, D>& L, const Prim<real, D>& R,
                                                  const real* __restrict__ waves, real* __restrict__ fluxBuf,
                                                  long long c) {
-    const int N = D + 2, E = N - 1;
+    const int N = D + 2;
     real sl = waves[((long long)SIDE * 2 + 0) * g.V + c];
     real sr = waves[((long long)SIDE * 2 + 1) * g.V + c];
-    real fL[N], fR[N], flux[N];
-    fL[0] = mulI(L.density, L.v[0]);
-    fL[1] = mulI(mulI(L.density, L.v[0]), L.v[0]) + L.pressure;
-#pragma unroll
-    for (int k = 1; k < D; ++k) fL[1 + k] = mulI(mulI(L.density, L.v[k]), L.v[0]);
-    fL[E] = mulI(mulI(L.density, L.enthalpyTotal), L.v[0]);
-    fR[0] = mulI(R.density, R.v[0]);
-    fR[1] = mulI(mulI(R.density, R.v[0]), R.v[0]) + R.pressure;
-#pragma unroll
-    for (int k = 1; k < D; ++k) fR[1 + k] = mulI(mulI(R.density, R.v[k]), R.v[0]);
-    fR[E] = mulI(mulI(R.density, R.enthalpyTotal), R.v[0]);
-    real sStar = divI(mulI(mulI(R.density, R.v[0]), sr - R.v[0]) - mulI(mulI(L.density, L.v[0]), sl - L.v[0]) +
-                          L.pressure - R.pressure,
-                      mulI(R.density, sr - R.v[0]) - mulI(L.density, sl - L.v[0]));
-    bool taken = true;
-    // (the branch tests on the bit patterns: double compares issue to the FP64 unit)
-    if (geZero(sl)) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) flux[i] = fL[i];
-    } else if (leZero(sl) && geZero(sStar)) {
-        real pressureLR = halfOf(L.pressure + R.pressure + mulI(mulI(L.density, sl - L.v[0]), sStar - L.v[0]) +
-                                 mulI(mulI(R.density, sr - R.v[0]), sStar - R.v[0]));
-        // every component divides by (sl - sStar)
-        const Divisor<real> den = divisorOf(sl - sStar);
-        flux[0] = quotBy(mulI(sStar, mulI(sl, stL[0]) - fL[0]), den);
-        flux[1] = quotBy(mulI(sStar, mulI(sl, stL[1]) - fL[1]) + mulI(sl, pressureLR), den);
-#pragma unroll
-        for (int k = 1; k < D; ++k) flux[1 + k] = quotBy(mulI(sStar, mulI(sl, stL[1 + k]) - fL[1 + k]), den);
-        flux[E] = quotBy(mulI(sStar, mulI(sl, stL[E]) - fL[E]) + mulI(mulI(sl, pressureLR), sStar), den);
-    } else if (leZero(sStar) && geZero(sr)) {
-        real pressureLR = halfOf(L.pressure + R.pressure + mulI(mulI(L.density, sl - L.v[0]), sStar - L.v[0]) +
-                                 mulI(mulI(R.density, sr - R.v[0]), sStar - R.v[0]));
-        const Divisor<real> den = divisorOf(sr - sStar);
-        flux[0] = quotBy(mulI(sStar, mulI(sr, stR[0]) - fR[0]), den);
-        flux[1] = quotBy(mulI(sStar, mulI(sr, stR[1]) - fR[1]) + mulI(sr, pressureLR), den);
-#pragma unroll
-        for (int k = 1; k < D; ++k) flux[1 + k] = quotBy(mulI(sStar, mulI(sr, stR[1 + k]) - fR[1 + k]), den);
-        flux[E] = quotBy(mulI(sStar, mulI(sr, stR[E]) - fR[E]) + mulI(mulI(sr, pressureLR), sStar), den);
-    } else if (leZero(sr)) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) flux[i] = fR[i];
-    } else {
+    real flux[N];
+    bool taken = true, done = false;
+    if constexpr (sizeof(real) == 8) {
+        if (ordinaryFace<D>(stL, stR, L, R, sl, sr)) {
+            CheckedOps o;
+            taken = hllcFluxOf(o, stL, stR, L, R, sl, sr, flux);
+            done = warpAll(o.ok);
+        }
+    }
+    if (!done) {
+        AnyOps<real> o;
+        taken = hllcFluxOf(o, stL, stR, L, R, sl, sr, flux);
+    }
+    if (!taken) {
         // no branch: the reference leaves the buffer's previous (global-frame) value,
         // then applies the rotate-back swap to it
-        taken = false;
 #pragma unroll
         for (int j = 0; j < N; ++j) flux[j] = fluxBuf[((long long)SIDE * N + j) * g.V + c];
     }
@@ -301,41 +369,44 @@ __device__ __forceinline__ bool hllFace(const Grid& g, const Phys<real>& ph, con
     return hllFaceFromPrim<real, D, SIDE>(g, stL, stR, L, R, waves, fluxBuf, c);
 }
 
+// the two-state HLL flux of one face (or one side's) into `flux`; false where no branch applies
+template <typename O, typename real, int D>
+__device__ __forceinline__ bool hllFluxOf(O& o, const real* stL, const real* stR, const Prim<real, D>& L,
+                                          const Prim<real, D>& R, real sl, real sr, real* flux) {
+    const int N = D + 2;
+    real fL[N], fR[N];
+    sideFlux(o, L, o.mul(L.density, L.v[0]), fL);
+    sideFlux(o, R, o.mul(R.density, R.v[0]), fR);
+    const bool left = geZero(sl), mid = leZero(sl) && geZero(sr), right = leZero(sr);
+    if (left || !mid) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) flux[i] = selectD(left, fL[i], fR[i]);
+    } else {
+        // FP32: `1. /` promotes; a double quotient rounded to float is the float quotient
+        const real invDenom = o.div((real)1, sr - sl);
+        const real slsr = o.mul(sl, sr);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const real t = o.mul(sr, fL[i]) - o.mul(sl, fR[i]) + o.mul(slsr, stR[i] - stL[i]);
+            flux[i] = o.mul(t, invDenom);
+        }
+    }
+    return left || mid || right;
+}
+
 // the rest of hllFace, given the face's rotated states and their primitives
 template <typename real, int D, int SIDE>
 __device__ __forceinline__ bool hllFaceFromPrim(const Grid& g, const real* stL, const real* stR,
                                                 const Prim<real, D>& L, const Prim<real, D>& R,
                                                 const real* __restrict__ waves, real* __restrict__ fluxBuf,
                                                 long long c) {
-    const int N = D + 2, E = N - 1;
+    const int N = D + 2;
     const real sl = waves[((long long)SIDE * 2 + 0) * g.V + c];
     const real sr = waves[((long long)SIDE * 2 + 1) * g.V + c];
-    real fL[N], fR[N], flux[N];
-    fL[0] = mulI(L.density, L.v[0]);
-    fL[1] = mulI(mulI(L.density, L.v[0]), L.v[0]) + L.pressure;
-#pragma unroll
-    for (int k = 1; k < D; ++k) fL[1 + k] = mulI(mulI(L.density, L.v[k]), L.v[0]);
-    fL[E] = mulI(mulI(L.density, L.enthalpyTotal), L.v[0]);
-    fR[0] = mulI(R.density, R.v[0]);
-    fR[1] = mulI(mulI(R.density, R.v[0]), R.v[0]) + R.pressure;
-#pragma unroll
-    for (int k = 1; k < D; ++k) fR[1 + k] = mulI(mulI(R.density, R.v[k]), R.v[0]);
-    fR[E] = mulI(mulI(R.density, R.enthalpyTotal), R.v[0]);
-    bool taken = true;
-    if (geZero(sl)) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) flux[i] = fL[i];
-    } else if (leZero(sl) && geZero(sr)) {
-        const real invDenom = (real)divI(1., (double)(sr - sl));
-        const real slsr = mulI(sl, sr);
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-            flux[i] = mulI(mulI(sr, fL[i]) - mulI(sl, fR[i]) + mulI(slsr, stR[i] - stL[i]), invDenom);
-    } else if (leZero(sr)) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) flux[i] = fR[i];
-    } else {
-        taken = false;                       // no branch: the previous (global-frame) value, swapped again
+    real flux[N];
+    AnyOps<real> o;      // (CheckedOps first, as hllcFaceFromPrim: 517x509 flux 55.4 -> 59.1 us)
+    const bool taken = hllFluxOf(o, stL, stR, L, R, sl, sr, flux);
+    if (!taken) {                                // no branch: the previous (global-frame) value, swapped again
 #pragma unroll
         for (int j = 0; j < N; ++j) flux[j] = fluxBuf[((long long)SIDE * N + j) * g.V + c];
     }
@@ -377,9 +448,16 @@ __device__ __forceinline__ bool hllcFluxCell(const Grid& g, const Phys<real>& ph
 
 // primitives of the tile's cells and of one cell below along every axis, into `prim`
 // (HX*HY*HZ entries, x fastest); the caller synchronises
-template <typename real, int D, bool GRAV>
+template <typename real, int D>
+__device__ __forceinline__ void stageRoots(Prim<real, D>&, double, bool) {}
+template <typename real, int D>
+__device__ __forceinline__ void stageRoots(WavePrim<real, D>& P, double gm1, bool hll) {
+    P.c = hll ? soundSpeed<true>(gm1, P) : soundSpeed<false>(gm1, P);
+    P.w = hll ? sqrtI(P.density) : (real)0;
+}
+template <typename real, int D, bool GRAV, bool HLL = false, typename P>
 __device__ __forceinline__ void stagePrims(const Grid& g, const Phys<real>& ph, const real* __restrict__ st,
-                                           int x0, int y0, int z0, int HX, int HY, int HZ, Prim<real, D>* prim,
+                                           int x0, int y0, int z0, int HX, int HY, int HZ, P* prim,
                                            const real* __restrict__ pot) {
     const int N = D + 2;
     const int ox = 1, oy = D > 1 ? 1 : 0, oz = D > 2 ? 1 : 0;
@@ -393,6 +471,7 @@ __device__ __forceinline__ void stagePrims(const Grid& g, const Phys<real>& ph, 
 #pragma unroll
                 for (int j = 0; j < N; ++j) s[j] = st[(long long)N * c + j];
                 primitives<real, D, GRAV>(s, ph.gamma, prim[i], GRAV ? pot[c] : (real)0);
+                stageRoots<real, D>(prim[i], (double)ph.gamma - 1., HLL);
             }
         }
     }
@@ -404,11 +483,11 @@ __device__ __forceinline__ void stagePrims(const Grid& g, const Phys<real>& ph, 
 template <typename real, int D, bool HLL = false, bool GRAV = false>
 __device__ __forceinline__ void hllcWaveTile(const Grid& g, const Phys<real>& ph, double gq,
                                              const real* __restrict__ state, real* __restrict__ waves, int x0, int y0,
-                                             int z0, int TX, int TY, int TZ, int s0, int s1, Prim<real, D>* prim,
+                                             int z0, int TX, int TY, int TZ, int s0, int s1, WavePrim<real, D>* prim,
                                              const real* __restrict__ pot = nullptr) {
     const int HX = TX + 1, HY = D > 1 ? TY + 1 : 1, HZ = D > 2 ? TZ + 1 : 1;
     const int ox = 1, oy = D > 1 ? 1 : 0, oz = D > 2 ? 1 : 0;
-    stagePrims<real, D, GRAV>(g, ph, state, x0, y0, z0, HX, HY, HZ, prim, pot);
+    stagePrims<real, D, GRAV, HLL>(g, ph, state, x0, y0, z0, HX, HY, HZ, prim, pot);
     __syncthreads();
     const int tx = threadIdx.x % TX, ty = (threadIdx.x / TX) % TY, tz = threadIdx.x / (TX * TY);
     const int x = x0 + tx, y = y0 + ty, z = z0 + tz;
@@ -416,30 +495,23 @@ __device__ __forceinline__ void hllcWaveTile(const Grid& g, const Phys<real>& ph
     if (tz < TZ && x < g.S[0] && y < g.S[1] && z < g.S[2] && slow >= s0 && slow < s1 && inRange(g, x, y, z, 2, 1)) {
         const long long c = x + (long long)g.S[0] * (y + (long long)g.S[1] * z);
         const int self = (tz + oz) * HY * HX + (ty + oy) * HX + (tx + ox);
-        const int below[3] = {1, HX, HX * HY};
-#pragma unroll
-        for (int side = 0; side < D; ++side) {
-            if (!cellOk(g, c) || !cellOk(g, c - g.step[side])) continue;
+        const double gm1 = (double)ph.gamma - 1.;
+        auto face = [&](auto sideTag, int below) {
+            constexpr int S = decltype(sideTag)::value;
+            if (!cellOk(g, c) || !cellOk(g, c - g.step[S])) return;
+            const WavePrim<real, D>&l = prim[self - below], &r = prim[self];
             Prim<real, D> L, R;
-            if (side == 0) {
-                rotatePrim<real, D, 0, GRAV>(prim[self - below[0]], ph.gamma, L);
-                rotatePrim<real, D, 0, GRAV>(prim[self], ph.gamma, R);
-                if (HLL) hllWaveFaceFromPrim<real, D, 0, GRAV>(g, ph, L, R, waves, c);
-                else waveFaceFromPrim<real, D, 0>(g, ph, gq, L, R, waves, c);
-            } else if (side == 1) {
-                constexpr int S1 = D > 1 ? 1 : 0;
-                rotatePrim<real, D, S1, GRAV>(prim[self - below[1]], ph.gamma, L);
-                rotatePrim<real, D, S1, GRAV>(prim[self], ph.gamma, R);
-                if (HLL) hllWaveFaceFromPrim<real, D, S1, GRAV>(g, ph, L, R, waves, c);
-                else waveFaceFromPrim<real, D, S1>(g, ph, gq, L, R, waves, c);
-            } else {
-                constexpr int S2 = D > 2 ? 2 : 0;
-                rotatePrim<real, D, S2, GRAV>(prim[self - below[2]], ph.gamma, L);
-                rotatePrim<real, D, S2, GRAV>(prim[self], ph.gamma, R);
-                if (HLL) hllWaveFaceFromPrim<real, D, S2, GRAV>(g, ph, L, R, waves, c);
-                else waveFaceFromPrim<real, D, S2>(g, ph, gq, L, R, waves, c);
-            }
-        }
+            rotatePrim<real, D, S, GRAV>(l, ph.gamma, L);
+            rotatePrim<real, D, S, GRAV>(r, ph.gamma, R);
+            // the rotation that re-forms |v|^2 and the enthalpy re-forms the sound speed
+            const bool again = D == 3 && S == 2;
+            const real cL = again ? soundSpeed<HLL>(gm1, L) : l.c, cR = again ? soundSpeed<HLL>(gm1, R) : r.c;
+            if (HLL) hllWaveFaceFromPrim<real, D, S, GRAV>(g, ph, L, R, cL, cR, l.w, r.w, waves, c);
+            else waveFaceFromPrim<real, D, S>(g, gq, L, R, cL, cR, waves, c);
+        };
+        face(std::integral_constant<int, 0>(), 1);
+        if (D > 1) face(std::integral_constant<int, (D > 1 ? 1 : 0)>(), HX);
+        if (D > 2) face(std::integral_constant<int, (D > 2 ? 2 : 0)>(), HX * HY);
     }
     __syncthreads();
 }
