@@ -103,7 +103,19 @@ __global__ void __launch_bounds__(kThreads) relaxKernel(Grid g, GravityConst<rea
         skewSum = skewSum + d;
     }
     // (4. * M_PI * G * density - skewSum) / diag, in double for both precisions
-    const real phi = (real)quotBy(rhs[c] - (double)skewSum, gc.diag);
+    const double rest = rhs[c] - (double)skewSum;
+    if constexpr (sizeof(real) == 8) {
+        // ordinary numbers in every lane: the quotients without a branch each
+        const double phi = quotPlain(rest, gc.diag);
+        if (warpAll(inWindow(rest) & inWindow(phi) & inWindow(gc.diag.b) & inWindow(gc.dxSq[0].b) &
+                    inWindow(gc.dxSq[D - 1].b) & inWindow(gc.dxSq[D / 2].b))) {
+#pragma unroll
+            for (int a = 0; a < (SAME ? 1 : D); ++a) quot[a * g.V + c] = quotPlain(phi, gc.dxSq[a]);
+            if (store) pot[c] = phi;
+            return;
+        }
+    }
+    const real phi = (real)quotBy(rest, gc.diag);
 #pragma unroll
     for (int a = 0; a < (SAME ? 1 : D); ++a) quot[a * g.V + c] = quotBy(phi, gc.dxSq[a]);
     if (store) pot[c] = phi;
