@@ -77,13 +77,15 @@ __global__ void __launch_bounds__(kThreads) hllcFluxKernel(Grid g, Phys<real> ph
 }
 
 // the flux with each cell's primitives staged once per tile (hllc_cells.cuh
-// hllcFluxTile), for slow-axis planes [s0, s1) (y in 2D, z in 3D)
+// hllcFluxTile), for slow-axis planes [s0, s1) (y in 2D, z in 3D).  Bound by the latency of
+// its integer chains: 2D at 3 blocks per SM (80 registers) 162 us a launch at 1021x1030, at 2
+// (110 registers) 182 us; 3D keeps 128 registers and 2 blocks.
 template <int D> struct FluxTile;
 template <> struct FluxTile<2> { enum { X = 32, Y = 8, Z = 1 }; };
 template <> struct FluxTile<3> { enum { X = 32, Y = 4, Z = 2 }; };
 
 template <typename real, int D, bool HLL, bool GRAV>
-__global__ void __launch_bounds__(kThreads) hllcFluxTileKernel(Grid g, Phys<real> ph, const real* __restrict__ stage,
+__global__ void __launch_bounds__(kThreads, D == 2 ? 3 : 2) hllcFluxTileKernel(Grid g, Phys<real> ph, const real* __restrict__ stage,
                                                                const real* __restrict__ waves,
                                                                real* __restrict__ flux, unsigned* health,
                                                                const real* __restrict__ pot, int s0, int s1) {
@@ -96,26 +98,6 @@ __global__ void __launch_bounds__(kThreads) hllcFluxTileKernel(Grid g, Phys<real
     const int z0 = D == 2 ? 0 : s0 + (int)blockIdx.z * T::Z;
     const bool ok = hllcFluxTile<real, D, HLL, GRAV>(g, ph, stage, waves, flux, x0, y0, z0, T::X, T::Y, T::Z, s0, s1,
                                                      prim, pot);
-    if (!ok) atomicOr(health, HEALTH_HLLC_NOBRANCH);
-}
-
-// The same for 2D EulerHLLC with the register budget of one block per SM: ptxas then
-// keeps 102 registers (2 blocks per SM) instead of its default 80 (3 blocks), which
-// measured faster (KH 2048^2 RK4 8.32 -> 7.71 ms a step); EulerHLL and 3D measured
-// slower that way and keep the kernel above.
-template <typename real, bool GRAV>
-__global__ void __launch_bounds__(kThreads, 1) hllcFluxTileKernelWide(Grid g, Phys<real> ph,
-                                                                      const real* __restrict__ stage,
-                                                                      const real* __restrict__ waves,
-                                                                      real* __restrict__ flux, unsigned* health,
-                                                                      const real* __restrict__ pot, int s0, int s1) {
-    dependentLaunch();
-    typedef FluxTile<2> T;
-    constexpr int HX = T::X + 1, HY = T::Y + 1;
-    __shared__ Prim<real, 2> prim[HX * HY];
-    const int x0 = blockIdx.x * T::X, y0 = s0 + (int)blockIdx.y * T::Y;
-    const bool ok = hllcFluxTile<real, 2, false, GRAV>(g, ph, stage, waves, flux, x0, y0, 0, T::X, T::Y, 1, s0, s1,
-                                                       prim, pot);
     if (!ok) atomicOr(health, HEALTH_HLLC_NOBRANCH);
 }
 
@@ -227,10 +209,7 @@ void launchHllcFluxG(const Grid& g, const Phys<real>& ph, const real* stage, con
             if (g.dim == 2) T(2, true)
             else T(3, true)
         } else {
-            if (g.dim == 2)
-                launchDependent(hllcFluxTileKernelWide<real, GRAV>, tileGrid<2>(g, s0, s1), kThreads, 0, st, g, ph, stage, waves,
-                                                                                                flux, health, pot, s0,
-                                                                                                s1);
+            if (g.dim == 2) T(2, false)
             else T(3, false)
         }
 #undef T

@@ -41,9 +41,11 @@ template <> struct BasisTile<1> { enum { X = 256, Y = 1, Z = 1 }; };
 template <> struct BasisTile<2> { enum { X = 32, Y = 8, Z = 1 }; };
 template <> struct BasisTile<3> { enum { X = 32, Y = 4, Z = 2 }; };
 
-// slowOff: tiles skipped along the slowest axis (y in 2D, z in 3D), for a band of it
+// slowOff: tiles skipped along the slowest axis (y in 2D, z in 3D), for a band of it.
+// 2D FP64 at 5 blocks per SM (KH 2048^2 525 -> 512 us a launch; FP32 and 3D are faster with
+// the registers they take, 106 against 109 us and 228 against 232)
 template <typename real, int D, bool GRAV>
-__global__ void __launch_bounds__(256) roeBasisKernel(Grid g, Phys<real> ph, const real* __restrict__ state,
+__global__ void __launch_bounds__(256, D == 2 && sizeof(real) == 8 ? 5 : 0) roeBasisKernel(Grid g, Phys<real> ph, const real* __restrict__ state,
                                                      real* __restrict__ basis, int loA, int hiA,
                                                      const real* __restrict__ pot, int slowOff) {
     dependentLaunch();
