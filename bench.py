@@ -557,21 +557,24 @@ MEASURED_TRAFFIC_PER_CELL = {"roe_flux": 568.0, "roe_delta_q_tilde": 252.0, "roe
 # Instructions the FP64 unit executes per interior cell of one launch of each kernel of
 # the EulerRoe FP64 step (MinMod), from ncu's smsp__inst_executed_pipe_fp64 (warp
 # instructions x 32) over the cells of the second of two KH 512x512 RK4 steps of the same
-# kernels; roe_flux is its two passes together (corrections 30.57 + transforms 65.55);
-# Delta-q-tilde and the combine vary by stage, so theirs are the step's means (Delta-q-
-# tilde 29.79 in every stage; the combine 40.87, 32.87, 32.87, 28.34).  763.1 per RK4
-# cell-update.
+# kernels; roe_flux is its two passes together; Delta-q-tilde and the combine vary by stage,
+# so theirs are the step's means.  FP64_PIPE_NOW is the current build's count (corrections
+# 29.79 + transforms 57.60; combine 32.93, 24.93, 24.93, 20.40; 627.8 per RK4 cell-update),
+# which the measurement uses; FP64_PIPE_PER_CELL an earlier build's (763.1), whose square
+# roots, quotient corrections and left rows ran on the FP64 unit.
+FP64_PIPE_NOW = {"roe_eigenbasis": 49.97, "cfl_min_reduce": 3.97, "roe_delta_q_tilde": 29.79,
+                 "roe_flux": 87.39, "flux_divergence_combine": 25.80, "state_check": 1.98}
 FP64_PIPE_PER_CELL = {"roe_eigenbasis": 112.62, "cfl_min_reduce": 9.92, "roe_delta_q_tilde": 29.79,
                       "roe_flux": 96.12, "flux_divergence_combine": 33.74, "state_check": 1.98}
 
 
-def fp64_roofline(prof, value, fp64_peak):
+def fp64_roofline(prof, value, fp64_peak, table=FP64_PIPE_PER_CELL):
     """The step's binding roofline: FP64-unit instructions per cell-update (the table
     above times each kernel's launches per step, from a profile of `steps` steps)
     times cell-updates/s, against the FP64 unit's issue rate measured in this run
     (hgpu_fp64_peak, FMA instructions per second on all SMs)."""
     steps = prof["roe_eigenbasis"][0] if "roe_eigenbasis" in prof else 1
-    per_update = sum(FP64_PIPE_PER_CELL.get(k, 0.) * v[0] / steps for k, v in prof.items())
+    per_update = sum(table.get(k, 0.) * v[0] / steps for k, v in prof.items())
     achieved = per_update * value
     return per_update, achieved, achieved / fp64_peak
 
@@ -656,7 +659,7 @@ def run_gb300(args):
     achieved_gbs = bytes_per_launch / (dom_ms * 1e-3) / 1e9
     fp64_peak = hg.fp64_peak()
     traffic = MEASURED_TRAFFIC_PER_CELL.get(dom_name)
-    per_update, fp64_achieved, fp64_frac = fp64_roofline(prof, value / world, fp64_peak)
+    per_update, fp64_achieved, fp64_frac = fp64_roofline(prof, value / world, fp64_peak, FP64_PIPE_NOW)
     step_bytes = 17 * N_STATES * 8          # compulsory bytes of an RK4 cell-update (17 state arrays)
     step_gbs = step_bytes * value / world / 1e9
     roofline = {"bound": "fp64", "kernel": "the whole step (each of its kernels is FP64-issue-bound)",
