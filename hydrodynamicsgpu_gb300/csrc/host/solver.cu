@@ -982,10 +982,10 @@ int Roe<real>::setFusedStages(bool on) {
 // not offered (ForwardEuler or FP32: a 2D FP64 Runge-Kutta stage stays the four kernels that
 // hgpu_set_fused_stages replaces by two), up to the size where the recomputed faces cost
 // more than the launches.  us a step, this path / the kernels for large grids: 1D RK2
-// Superbee FP64 1028 cells 32.8 / 47.2, 65536 49 / 78, 262144 121 / 129, 2^20 446 / 434
-// (FP32 16 / 25, 20 / 29, 45 / 42, 143 / 106); 2D ForwardEuler FP64 64^2 35 / 66, 181^2
-// 66 / 69, 256^2 108 / 86; 2D RK2 FP32 64^2 19 / 35, 256^2 33 / 41, 362^2 48 / 49, 512^2
-// 76 / 61.
+// Superbee FP64 1028 cells 28 / 39, 65536 43 / 66 (FP32 16 / 25, 21 / 29); 2D ForwardEuler
+// FP64 64^2 31 / 55, 181^2 56 / 60; 2D RK2 FP32 64^2 19 / 33, 256^2 33 / 39.  Past the lines,
+// when the path was made: 1D 2^20 446 / 434 (FP32 262144 45 / 42), ForwardEuler 256^2
+// 108 / 86, FP32 512^2 76 / 61.
 template <typename real>
 bool Roe<real>::smallGrid() const {
     const auto& c = this->rc.cfg;

@@ -1,8 +1,8 @@
 // roe_small.cu -- EulerRoe steps of small grids in few launches (sm_103a).
 //
 // On a small grid a step's kernels are all latency: a launch holds a few warps on a few
-// SMs, and the step pays its chain of launches (12 for a 1D RungeKutta2 step, 48 us at 1028
-// cells, of which the FP64 unit needs 0.3 us).  Here the step is one prologue kernel, one
+// SMs, and the step pays its chain of launches (12 for a 1D RungeKutta2 step, 39 us at 1028
+// cells against 28 here, of which the FP64 unit needs 0.3 us).  Here the step is one prologue kernel, one
 // kernel a stage and, for ForwardEuler, one to finish; a block takes a small tile, so that
 // a grid of a thousand cells is spread over tens of SMs, and recomputes the faces that its
 // neighbours also need instead of waiting for them:
