@@ -196,8 +196,8 @@ __device__ __forceinline__ void stageCotangent(const AdjStage& st, long long c, 
 // measured 0.996 ms per backward step against 0.998 with 3 and 1.008 uncapped)
 template <int D>
 __global__ void __launch_bounds__(kT, 4) adjFluxKernel(Grid g, Phys<double> ph, int lim, double k0, double k1, double k2,
-                                                    const double* __restrict__ U, const double* __restrict__ DQ,
-                                                    const double* __restrict__ B, const double* __restrict__ FT,
+                                                    const double* U, const double* DQ,
+                                                    const double* B, const double* FT,
                                                     AdjStage st, AdjScratch S, int first) {
     dependentLaunch();
     const int N = D + 2;
@@ -256,8 +256,8 @@ __device__ __forceinline__ void adjDeltaQFace(const Grid& g, double gm1, const d
 }
 
 template <int D>
-__global__ void __launch_bounds__(kT) adjDeltaQKernel(Grid g, Phys<double> ph, const double* __restrict__ U,
-                                                      const double* __restrict__ B, AdjScratch S) {
+__global__ void __launch_bounds__(kT) adjDeltaQKernel(Grid g, Phys<double> ph, const double* U,
+                                                      const double* B, AdjScratch S) {
     dependentLaunch();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
@@ -363,7 +363,7 @@ __device__ __forceinline__ void adjBasisFace(const Grid& g, const Phys<double>& 
 }
 
 template <int D>
-__global__ void __launch_bounds__(kT) adjBasisKernel(Grid g, Phys<double> ph, const double* __restrict__ U,
+__global__ void __launch_bounds__(kT) adjBasisKernel(Grid g, Phys<double> ph, const double* U,
                                                      AdjScratch S) {
     dependentLaunch();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -378,8 +378,8 @@ __global__ void __launch_bounds__(kT) adjBasisKernel(Grid g, Phys<double> ph, co
 // (v..., h, w) cotangents of a cell -> its conserved state, added to lam
 //   v_k = m_k / rho,  h = gamma E / rho - (gamma - 1) .5 |v|^2,  w = sqrt(rho)
 template <int D>
-__global__ void __launch_bounds__(kT) adjPrimsKernel(Grid g, Phys<double> ph, const double* __restrict__ U,
-                                                     AdjScratch S, double* __restrict__ lam) {
+__global__ void __launch_bounds__(kT) adjPrimsKernel(Grid g, Phys<double> ph, const double* U,
+                                                     AdjScratch S, double* lam) {
     dependentLaunch();
     const int N = D + 2, P = D + 2, E = N - 1;
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kT) adjPrimsKernel(Grid g, Phys<double> ph, co
 }
 
 // transposed ghost fill of one line along `axis` (boundaryLine run backwards)
-__global__ void adjBoundaryKernel(Grid g, int axis, int N, int mMin, int mMax, double* __restrict__ lam) {
+__global__ void adjBoundaryKernel(Grid g, int axis, int N, int mMin, int mMax, double* lam) {
     dependentLaunch();
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int A = axis == 0 ? 1 : 0, B = axis == 2 ? 1 : 2;

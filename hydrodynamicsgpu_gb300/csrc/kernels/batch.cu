@@ -23,7 +23,7 @@ namespace {
 // ghost fill of one problem per work item: every axis in order, lines in parallel
 template <typename real, int D>
 __global__ void __launch_bounds__(256) batchBoundaryKernel(const BatchProblem<real>* __restrict__ P, int nP,
-                                                           real* __restrict__ state, unsigned* q) {
+                                                           real* state, unsigned* q) {
     dependentLaunch();
     for (;;) {
         int p = nextItem(q);
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(256) batchBoundaryKernel(const BatchProblem<re
 template <typename real, int D, bool PLAIN>
 __global__ void __launch_bounds__(256) batchRoeBasisKernel(const BatchProblem<real>* __restrict__ P,
                                                            const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
-                                                           int loA, int hiA, const real* __restrict__ state,
+                                                           int loA, int hiA, const real* state,
                                                            real* __restrict__ basis, unsigned* q) {
     dependentLaunch();
     extern __shared__ unsigned char smem[];
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256) batchRoeBasisKernel(const BatchProblem<re
 template <typename real, int D, bool PLAIN>
 __global__ void __launch_bounds__(256) batchDtKernel(const BatchProblem<real>* __restrict__ P,
                                                      const BatchTile* __restrict__ tiles, int nT, BatchTuning tu, int hllc,
-                                                     const real* __restrict__ faces, unsigned long long* acc,
+                                                     const real* faces, unsigned long long* acc,
                                                      unsigned* health, unsigned* q) {
     dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
@@ -118,8 +118,8 @@ __global__ void batchFinalizeKernel(const BatchProblem<real>* __restrict__ P, in
 template <typename real, int D, bool PLAIN>
 __global__ void __launch_bounds__(256) batchDeltaQKernel(const BatchProblem<real>* __restrict__ P,
                                                          const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
-                                                         int loA, int hiA, const real* __restrict__ stage,
-                                                         const real* __restrict__ basis, real* __restrict__ dq,
+                                                         int loA, int hiA, const real* stage,
+                                                         const real* basis, real* __restrict__ dq,
                                                          unsigned* q) {
     dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(256) batchDeltaQKernel(const BatchProblem<real
 template <typename real, int D, bool PLAIN>
 __global__ void __launch_bounds__(256, PLAIN ? 5 : 1) batchCombineKernel(const BatchProblem<real>* __restrict__ P,
                                                           const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
-                                                          const real* __restrict__ flux, CombinePlan<real> plan,
-                                                          const StepConst<real>* __restrict__ sc, unsigned* q) {
+                                                          const real* flux, CombinePlan<real> plan,
+                                                          const StepConst<real>* sc, unsigned* q) {
     dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
         const BatchTile tl = tiles[t];
@@ -159,8 +159,8 @@ __global__ void __launch_bounds__(256, PLAIN ? 5 : 1) batchCombineKernel(const B
 template <typename real, int D>
 __global__ void __launch_bounds__(256) batchGravityKernel(const BatchProblem<real>* __restrict__ P,
                                                           const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
-                                                          int integ, const StepConst<real>* __restrict__ sc,
-                                                          real* __restrict__ state, unsigned* q) {
+                                                          int integ, const StepConst<real>* sc,
+                                                          real* state, unsigned* q) {
     dependentLaunch();
     for (int t = firstItem(q, tu); t < nT; t = nextItemAfter(q, tu)) {
         const BatchTile tl = tiles[t];
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) batchGravityKernel(const BatchProblem<rea
 template <typename real, int D, bool PLAIN>
 __global__ void __launch_bounds__(256) batchStateCheckKernel(const BatchProblem<real>* __restrict__ P,
                                                              const BatchTile* __restrict__ tiles, int nT,
-                                                             BatchTuning tu, const real* __restrict__ state,
+                                                             BatchTuning tu, const real* state,
                                                              unsigned* health, unsigned* healthP, unsigned* q) {
     dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(256) batchStateCheckKernel(const BatchProblem<
 template <typename real, int D, bool HLL>
 __global__ void __launch_bounds__(256) batchWaveKernel(const BatchProblem<real>* __restrict__ P,
                                                        const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
-                                                       const real* __restrict__ state, real* __restrict__ waves,
+                                                       const real* state, real* __restrict__ waves,
                                                        unsigned* q) {
     dependentLaunch();
     for (int t = firstItem(q, tu); t < nT; t = nextItemAfter(q, tu)) {

@@ -16,9 +16,9 @@ namespace {
 template <typename real, int D, int HLLC, int LIM>
 __global__ void __launch_bounds__(256) batchFluxKernel(const BatchProblem<real>* __restrict__ P,
                                                        const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
-                                                       int hllc, int lim, const StepConst<real>* __restrict__ sc,
-                                                       const real* __restrict__ stage, const real* __restrict__ faces,
-                                                       const real* __restrict__ dq, real* __restrict__ flux,
+                                                       int hllc, int lim, const StepConst<real>* sc,
+                                                       const real* stage, const real* faces,
+                                                       const real* dq, real* flux,
                                                        unsigned* health, unsigned* q) {
     dependentLaunch();
     for (int t = firstItem(q, tu); t < nT; t = nextItemAfter(q, tu)) {
@@ -49,9 +49,9 @@ __global__ void __launch_bounds__(256) batchFluxKernel(const BatchProblem<real>*
 template <int D, int LIM, bool PLAIN>
 __global__ void __launch_bounds__(256) batchFluxCorrKernel(const BatchProblem<double>* __restrict__ P,
                                                            const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
-                                                           int lim, const StepConst<double>* __restrict__ sc,
-                                                           const double* __restrict__ faces,
-                                                           const double* __restrict__ dq, double* __restrict__ flux,
+                                                           int lim, const StepConst<double>* sc,
+                                                           const double* faces,
+                                                           const double* dq, double* __restrict__ flux,
                                                            unsigned* q) {
     dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
@@ -72,9 +72,9 @@ __global__ void __launch_bounds__(256) batchFluxCorrKernel(const BatchProblem<do
 template <int D, bool PLAIN>
 __global__ void __launch_bounds__(256, PLAIN && D <= 2 ? 3 : 1) batchFluxXformKernel(const BatchProblem<double>* __restrict__ P,
                                                             const BatchTile* __restrict__ tiles, int nT, BatchTuning tu,
-                                                            const double* __restrict__ stage,
-                                                            const double* __restrict__ faces,
-                                                            double* __restrict__ flux, unsigned* q) {
+                                                            const double* stage,
+                                                            const double* faces,
+                                                            double* flux, unsigned* q) {
     dependentLaunch();
     for (int t = firstTile<PLAIN>(q); t < nT; t = nextTile<PLAIN>(q, nT)) {
         const BatchTile tl = tiles[t];

@@ -39,7 +39,7 @@ inline unsigned blocksFor(long long n) { return (unsigned)((n + kThreads - 1) / 
 // (a ghost is copied from a ghost filled before it)
 template <typename real>
 __global__ void __launch_bounds__(kThreads) boundaryKernel(Grid g, int axis, int N, int mMin, int mMax,
-                                                           real* __restrict__ state, long long t0, long long t1) {
+                                                           real* state, long long t0, long long t1) {
     dependentLaunch();
     const long long t = t0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= t1) return;
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(kThreads) boundaryKernel(Grid g, int axis, int
 // one axis, one thread a ghost cell: thread (line t, k-th of the line's four ghosts)
 template <typename real>
 __global__ void __launch_bounds__(kThreads) ghostAxisKernel(Grid g, int axis, int N, int mMin, int mMax,
-                                                            real* __restrict__ state, long long t0, long long t1) {
+                                                            real* state, long long t0, long long t1) {
     dependentLaunch();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, t = t0 + i / 4;
     if (t >= t1) return;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kThreads) ghostAxisKernel(Grid g, int axis, in
 // side by side, every copy after the one before) took 15 us at 133 x 97 and 17 us at
 // 2048^2 for the two launches; this one 6 us at both (event-timed, launch included).
 template <typename real>
-__global__ void __launch_bounds__(kThreads) ghostKernel(Grid g, int N, Methods bc, real* __restrict__ state,
+__global__ void __launch_bounds__(kThreads) ghostKernel(Grid g, int N, Methods bc, real* state,
                                                         long long n0, long long n1, long long n) {
     dependentLaunch();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -107,9 +107,9 @@ __global__ void __launch_bounds__(kThreads) ghostKernel(Grid g, int N, Methods b
 // the last stage (as a pass of its own over the state: 3D 160x144x136 RungeKutta2TVD 482 us
 // of the step, 3D 99x90x86 RungeKutta3TVD 211 us; folded, 60 and 55 us more of combine)
 template <typename real, int D, bool POST>
-__global__ void __launch_bounds__(kThreads, D < 3 || sizeof(real) == 4 ? 5 : 4) derivCombineKernel(Grid g, Phys<real> ph, const real* __restrict__ flux,
+__global__ void __launch_bounds__(kThreads, D < 3 || sizeof(real) == 4 ? 5 : 4) derivCombineKernel(Grid g, Phys<real> ph, const real* flux,
                                                                CombinePlan<real> plan,
-                                                               const StepConst<real>* __restrict__ sc, long long c0,
+                                                               const StepConst<real>* sc, long long c0,
                                                                long long c1) {
     dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -120,8 +120,8 @@ __global__ void __launch_bounds__(kThreads, D < 3 || sizeof(real) == 4 ? 5 : 4) 
 }
 
 template <typename real>
-__global__ void __launch_bounds__(kThreads) alphaOnlyKernel(long long n, int integ, real* __restrict__ state,
-                                                            const StepConst<real>* __restrict__ sc) {
+__global__ void __launch_bounds__(kThreads) alphaOnlyKernel(long long n, int integ, real* state,
+                                                            const StepConst<real>* sc) {
     dependentLaunch();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -138,8 +138,8 @@ __global__ void fixedDtKernel(Phys<real> ph, int integ, double fixedDt, StepCons
 // Self-gravity pass with ForwardEuler and a zero potential: the (ghost-refreshed)
 // state gets `state + deriv * dt` with deriv == +0 (ForwardEuler.cpp:20-32).
 template <typename real>
-__global__ void __launch_bounds__(kThreads) zeroAddKernel(long long n, real* __restrict__ state,
-                                                          const StepConst<real>* __restrict__ sc) {
+__global__ void __launch_bounds__(kThreads) zeroAddKernel(long long n, real* state,
+                                                          const StepConst<real>* sc) {
     dependentLaunch();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;

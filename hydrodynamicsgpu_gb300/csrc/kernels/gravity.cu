@@ -34,8 +34,8 @@ inline unsigned blocksFor(long long n) { return (unsigned)((n + kThreads - 1) / 
 
 // potential = -density (useGravity) or the given channel; total energy += that potential
 template <typename real, int D>
-__global__ void __launch_bounds__(kThreads) potentialInitKernel(Grid g, int fromDensity, real* __restrict__ state,
-                                                                real* __restrict__ pot, long long c0, long long c1) {
+__global__ void __launch_bounds__(kThreads) potentialInitKernel(Grid g, int fromDensity, real* state,
+                                                                real* pot, long long c0, long long c1) {
     dependentLaunch();
     const long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kThreads) potentialInitKernel(Grid g, int from
 // the potential's ghost fill along one axis: boundaryLine on a one-component buffer
 template <typename real>
 __global__ void __launch_bounds__(kThreads) potentialBoundaryKernel(Grid g, int axis, int mMin, int mMax,
-                                                                    real* __restrict__ pot) {
+                                                                    real* pot) {
     dependentLaunch();
     boundaryLine<real>(g, axis, 1, mMin, mMax, pot, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kThreads) potentialBoundaryKernel(Grid g, int 
 // cell instead of the state's record
 template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) relaxRhsKernel(Grid g, GravityConst<real> gc,
-                                                           const real* __restrict__ state, double* __restrict__ rhs) {
+                                                           const real* state, double* __restrict__ rhs) {
     dependentLaunch();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
@@ -78,8 +78,8 @@ __global__ void __launch_bounds__(kThreads) relaxRhsKernel(Grid g, GravityConst<
 // the quotients' integer work.
 template <typename real, int D, bool SAME, bool FIRST>
 __global__ void __launch_bounds__(kThreads) relaxKernel(Grid g, GravityConst<real> gc, int colour, bool store,
-                                                        const double* __restrict__ rhs, real* __restrict__ quot,
-                                                        real* __restrict__ pot) {
+                                                        const double* rhs, real* quot,
+                                                        real* pot) {
     dependentLaunch();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = D > 1 ? (int)blockIdx.y + 2 : 0, z = D > 2 ? (int)blockIdx.z + 2 : 0;
@@ -124,9 +124,9 @@ __global__ void __launch_bounds__(kThreads) relaxKernel(Grid g, GravityConst<rea
 // calcGravityDeriv of one cell into d (zero outside the interior), then the combine
 template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) gravityCombineKernel(Grid g, GravityConst<real> gc,
-                                                                 const real* __restrict__ stage,
-                                                                 const real* __restrict__ pot, CombinePlan<real> plan,
-                                                                 const StepConst<real>* __restrict__ sc) {
+                                                                 const real* stage,
+                                                                 const real* pot, CombinePlan<real> plan,
+                                                                 const StepConst<real>* sc) {
     dependentLaunch();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;

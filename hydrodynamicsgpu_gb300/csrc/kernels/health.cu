@@ -10,8 +10,8 @@ namespace {
 constexpr int kThreads = 256;
 
 template <typename real, int D>
-__global__ void __launch_bounds__(kThreads) stateCheckKernel(Grid g, const real* __restrict__ state,
-                                                             const real* __restrict__ pot, unsigned* health) {
+__global__ void __launch_bounds__(kThreads) stateCheckKernel(Grid g, const real* state,
+                                                             const real* pot, unsigned* health) {
     dependentLaunch();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned bits = 0;

@@ -27,8 +27,8 @@ inline unsigned blocksFor(long long n) { return (unsigned)((n + kThreads - 1) / 
 
 template <typename real, int D, bool HLL, bool GRAV>
 __global__ void __launch_bounds__(kThreads) hllcWaveKernel(Grid g, Phys<real> ph, double gq,
-                                                           const real* __restrict__ state, real* __restrict__ waves,
-                                                           const real* __restrict__ pot, long long c0, long long c1) {
+                                                           const real* state, real* __restrict__ waves,
+                                                           const real* pot, long long c0, long long c1) {
     dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;
@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(kThreads) hllcWaveKernel(Grid g, Phys<real> ph
 inline unsigned cflBlocks(long long n) { return std::min(blocksFor(n), 152u * 8u); }
 
 template <typename real, int D>
-__global__ void __launch_bounds__(kThreads) hllcDtKernel(Grid g, Phys<real> ph, const real* __restrict__ waves, int integ,
+__global__ void __launch_bounds__(kThreads) hllcDtKernel(Grid g, Phys<real> ph, const real* waves, int integ,
                                                         unsigned long long accInit, CflAcc* acc, StepConst<real>* sc) {
     dependentLaunch();
     unsigned long long s[D] = {};
@@ -63,9 +63,9 @@ __global__ void __launch_bounds__(kThreads) hllcDtKernel(Grid g, Phys<real> ph, 
 }
 
 template <typename real, int D, bool HLL, bool GRAV>
-__global__ void __launch_bounds__(kThreads) hllcFluxKernel(Grid g, Phys<real> ph, const real* __restrict__ stage,
-                                                           const real* __restrict__ waves, real* __restrict__ flux,
-                                                           unsigned* health, const real* __restrict__ pot,
+__global__ void __launch_bounds__(kThreads) hllcFluxKernel(Grid g, Phys<real> ph, const real* stage,
+                                                           const real* waves, real* flux,
+                                                           unsigned* health, const real* pot,
                                                            long long c0, long long c1) {
     dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -85,10 +85,10 @@ template <> struct FluxTile<2> { enum { X = 32, Y = 8, Z = 1 }; };
 template <> struct FluxTile<3> { enum { X = 32, Y = 4, Z = 2 }; };
 
 template <typename real, int D, bool HLL, bool GRAV>
-__global__ void __launch_bounds__(kThreads, D == 2 ? 3 : 2) hllcFluxTileKernel(Grid g, Phys<real> ph, const real* __restrict__ stage,
-                                                               const real* __restrict__ waves,
-                                                               real* __restrict__ flux, unsigned* health,
-                                                               const real* __restrict__ pot, int s0, int s1) {
+__global__ void __launch_bounds__(kThreads, D == 2 ? 3 : 2) hllcFluxTileKernel(Grid g, Phys<real> ph, const real* stage,
+                                                               const real* waves,
+                                                               real* flux, unsigned* health,
+                                                               const real* pot, int s0, int s1) {
     dependentLaunch();
     typedef FluxTile<D> T;
     constexpr int HX = T::X + 1, HY = T::Y + 1, HZ = D > 2 ? T::Z + 1 : 1;
@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(kThreads, D == 2 ? 3 : 2) hllcFluxTileKernel(G
 
 template <typename real, int D, bool HLL, bool GRAV>
 __global__ void __launch_bounds__(kThreads) hllcWaveTileKernel(Grid g, Phys<real> ph, double gq,
-                                                               const real* __restrict__ state,
-                                                               real* __restrict__ waves, const real* __restrict__ pot,
+                                                               const real* state,
+                                                               real* __restrict__ waves, const real* pot,
                                                                int s0, int s1) {
     dependentLaunch();
     typedef FluxTile<D> T;

@@ -8,6 +8,15 @@
 // let the next grid start in turn, then wait until the previous grid has completed and its
 // writes are visible.  Nothing is read or written before that wait, so the order of memory
 // operations is that of plain launches.
+//
+// What keeps the compiler to that order: the wait is a volatile asm with a "memory" clobber,
+// which binds every access to memory that may have other names.  A pointer parameter that is
+// `__restrict__` is taken to have none, and one that is also `const` lets its loads be issued as
+// read-only for the kernel's whole life (ld.global.nc), which starts before the wait while
+// earlier kernels still write.  So these kernels declare `__restrict__` only what they write
+// and do not read, and the tables that the host fills when a batch is made.  It costs nothing
+// measurable: with `const __restrict__` inputs the steps of 2048^2, 1024^2, 160x144x136 and of
+// the 1D shock tube took the same within 0.2 %.
 #pragma once
 #include <cuda_runtime.h>
 

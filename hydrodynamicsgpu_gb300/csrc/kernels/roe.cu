@@ -45,9 +45,9 @@ template <> struct BasisTile<3> { enum { X = 32, Y = 4, Z = 2 }; };
 // 2D FP64 at 5 blocks per SM (KH 2048^2 525 -> 512 us a launch; FP32 and 3D are faster with
 // the registers they take, 106 against 109 us and 228 against 232)
 template <typename real, int D, bool GRAV>
-__global__ void __launch_bounds__(256, D == 2 && sizeof(real) == 8 ? 5 : 0) roeBasisKernel(Grid g, Phys<real> ph, const real* __restrict__ state,
+__global__ void __launch_bounds__(256, D == 2 && sizeof(real) == 8 ? 5 : 0) roeBasisKernel(Grid g, Phys<real> ph, const real* state,
                                                      real* __restrict__ basis, int loA, int hiA,
-                                                     const real* __restrict__ pot, int slowOff) {
+                                                     const real* pot, int slowOff) {
     dependentLaunch();
     typedef BasisTile<D> T;
     constexpr int HX = T::X + 1, HY = D > 1 ? T::Y + 1 : 1, HZ = D > 2 ? T::Z + 1 : 1;
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256, D == 2 && sizeof(real) == 8 ? 5 : 0) roeB
 inline unsigned cflBlocks(long long n) { return std::min(blocksFor(n), 152u * 8u); }
 
 template <typename real, int D>
-__global__ void __launch_bounds__(kThreads) roeDtKernel(Grid g, Phys<real> ph, const real* __restrict__ basis, int integ,
+__global__ void __launch_bounds__(kThreads) roeDtKernel(Grid g, Phys<real> ph, const real* basis, int integ,
                                                         unsigned long long accInit, CflAcc* acc, StepConst<real>* sc) {
     dependentLaunch();
     unsigned long long s[D] = {};
@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(kThreads) roeDtKernel(Grid g, Phys<real> ph, c
 }
 
 template <typename real, int D>
-__global__ void __launch_bounds__(kStageThreads, D < 3 ? 8 : 6) roeDeltaQKernel(Grid g, const real* __restrict__ stage,
-                                                            const real* __restrict__ basis, real* __restrict__ dq,
+__global__ void __launch_bounds__(kStageThreads, D < 3 ? 8 : 6) roeDeltaQKernel(Grid g, const real* stage,
+                                                            const real* basis, real* __restrict__ dq,
                                                             int loA, int hiA, long long c0, long long c1) {
     dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -95,9 +95,9 @@ __global__ void __launch_bounds__(kStageThreads, D < 3 ? 8 : 6) roeDeltaQKernel(
 }
 
 template <typename real, int D, int LIM>
-__global__ void __launch_bounds__(kThreads) roeFluxKernel(Grid g, int lim, const real* __restrict__ stage,
-                                                          const real* __restrict__ basis, const real* __restrict__ dq,
-                                                          const StepConst<real>* __restrict__ sc,
+__global__ void __launch_bounds__(kThreads) roeFluxKernel(Grid g, int lim, const real* stage,
+                                                          const real* basis, const real* dq,
+                                                          const StepConst<real>* sc,
                                                           real* __restrict__ flux, long long c0, long long c1) {
     dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -108,9 +108,9 @@ __global__ void __launch_bounds__(kThreads) roeFluxKernel(Grid g, int lim, const
 }
 
 template <int D, int LIM>
-__global__ void __launch_bounds__(kStageThreads, D < 3 ? 8 : 6) roeFluxCorrKernel(Grid g, int lim, const double* __restrict__ basis,
-                                                              const double* __restrict__ dq,
-                                                              const StepConst<double>* __restrict__ sc,
+__global__ void __launch_bounds__(kStageThreads, D < 3 ? 8 : 6) roeFluxCorrKernel(Grid g, int lim, const double* basis,
+                                                              const double* dq,
+                                                              const StepConst<double>* sc,
                                                               double* __restrict__ flux, long long c0, long long c1) {
     dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -121,9 +121,9 @@ __global__ void __launch_bounds__(kStageThreads, D < 3 ? 8 : 6) roeFluxCorrKerne
 }
 
 template <int D>
-__global__ void __launch_bounds__(kStageThreads, D < 3 ? 6 : 4) roeFluxXformKernel(Grid g, const double* __restrict__ stage,
-                                                               const double* __restrict__ basis,
-                                                               double* __restrict__ flux, long long c0, long long c1) {
+__global__ void __launch_bounds__(kStageThreads, D < 3 ? 6 : 4) roeFluxXformKernel(Grid g, const double* stage,
+                                                               const double* basis,
+                                                               double* flux, long long c0, long long c1) {
     dependentLaunch();
     long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= c1) return;

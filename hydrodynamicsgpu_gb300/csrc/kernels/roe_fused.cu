@@ -49,8 +49,8 @@ static_assert(kRows == 8, "the y pass's ring indexing assumes 8 rows per step");
 // ---------------- x pass ----------------
 template <int LIM>
 __global__ void __launch_bounds__(kThreadsX, kBlocksX)
-    roeStageXKernel(Grid g, Phys<double> ph, int lim, const StepConst<double>* __restrict__ sc,
-                    const double* __restrict__ stage, const double* __restrict__ basis, double* __restrict__ dX,
+    roeStageXKernel(Grid g, Phys<double> ph, int lim, const StepConst<double>* sc,
+                    const double* stage, const double* basis, double* __restrict__ dX,
                     int loA, int hiA, unsigned* health) {
     dependentLaunch();
     constexpr int N = 4, NB = RoeRec<2>::NB;
@@ -155,8 +155,8 @@ __device__ __forceinline__ double* fRow(YShared& sm, int f, int r0) {
 
 template <int LIM>
 __global__ void __launch_bounds__(kThreads, 3)
-    roeStageYKernel(Grid g, Phys<double> ph, int lim, const StepConst<double>* __restrict__ sc,
-                    const double* __restrict__ basis, const double* __restrict__ dX, CombinePlan<double> plan,
+    roeStageYKernel(Grid g, Phys<double> ph, int lim, const StepConst<double>* sc,
+                    const double* basis, const double* dX, CombinePlan<double> plan,
                     const __grid_constant__ CUtensorMap tm, int loA, int hiA, unsigned* health) {
     dependentLaunch();
     constexpr int N = 4, NB = RoeRec<2>::NB;

@@ -15,9 +15,9 @@ constexpr int kThreads = 256;
 // (recording A, phi, phi', r), then the transforms (recording L avg and ft)
 template <int D, int LIM>
 __global__ void __launch_bounds__(kThreads) roeFluxCorrRecordKernel(Grid g, int lim,
-                                                                    const double* __restrict__ basis,
-                                                                    const double* __restrict__ dq,
-                                                                    const StepConst<double>* __restrict__ sc,
+                                                                    const double* basis,
+                                                                    const double* dq,
+                                                                    const StepConst<double>* sc,
                                                                     double* __restrict__ flux,
                                                                     double* __restrict__ tape) {
     dependentLaunch();
@@ -29,9 +29,9 @@ __global__ void __launch_bounds__(kThreads) roeFluxCorrRecordKernel(Grid g, int 
 }
 
 template <int D>
-__global__ void __launch_bounds__(kThreads) roeFluxXformRecordKernel(Grid g, const double* __restrict__ stage,
-                                                                     const double* __restrict__ basis,
-                                                                     double* __restrict__ flux,
+__global__ void __launch_bounds__(kThreads) roeFluxXformRecordKernel(Grid g, const double* stage,
+                                                                     const double* basis,
+                                                                     double* flux,
                                                                      double* __restrict__ tape) {
     dependentLaunch();
     long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -114,8 +114,8 @@ __global__ void __launch_bounds__(SmallTile<D>::THREADS) smallPrologueKernel(Gri
 
 template <typename real, int D, int LIM, bool POST>
 __global__ void __launch_bounds__(SmallTile<D>::THREADS) smallStageKernel(Grid g, Phys<real> ph, int lim,
-                                                                       const StepConst<real>* __restrict__ sc,
-                                                                       const real* __restrict__ basis,
+                                                                       const StepConst<real>* sc,
+                                                                       const real* basis,
                                                                        CombinePlan<real> plan) {
     dependentLaunch();
     typedef SmallTile<D> T;
@@ -210,9 +210,9 @@ __global__ void __launch_bounds__(SmallTile<D>::THREADS) smallStageKernel(Grid g
 // ForwardEuler's end (the self-gravity pass with a zero potential): the updated state out of
 // `next`, ghosts from where the ghost fill copies them, + 0 * dt
 template <typename real>
-__global__ void __launch_bounds__(64) smallFinishKernel(Grid g, int N, Methods bc, const real* __restrict__ next,
-                                                        real* __restrict__ state,
-                                                        const StepConst<real>* __restrict__ sc) {
+__global__ void __launch_bounds__(64) smallFinishKernel(Grid g, int N, Methods bc, const real* next,
+                                                        real* state,
+                                                        const StepConst<real>* sc) {
     dependentLaunch();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.V) return;
