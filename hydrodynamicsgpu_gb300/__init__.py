@@ -69,6 +69,7 @@ SIGNATURES = {
     "hgpu_limiter_selftest": (ctypes.c_int, [ctypes.c_ulonglong, ctypes.c_longlong, ctypes.POINTER(ctypes.c_longlong)]),
     "hgpu_fp64_selftest": (ctypes.c_int, [ctypes.c_ulonglong, ctypes.c_longlong, ctypes.POINTER(ctypes.c_longlong),
                                           ctypes.POINTER(ctypes.c_longlong)]),
+    "hgpu_arith_selftest": (ctypes.c_int, [ctypes.c_ulonglong, ctypes.c_longlong, ctypes.POINTER(ctypes.c_longlong)]),
     "hgpu_display": (ctypes.c_int, [_P, ctypes.c_int, ctypes.POINTER(ctypes.c_float), ctypes.c_size_t]),
     "hgpu_display_device": (ctypes.c_int, [_P, ctypes.c_int, _P]),
     "hgpu_save_fits": (ctypes.c_int, [_P, ctypes.c_char_p, ctypes.POINTER(ctypes.c_int)]),
@@ -117,6 +118,14 @@ def fp64_selftest(cases=1 << 26, seed=1):
     m, d = ctypes.c_longlong(), ctypes.c_longlong()
     check(lib().hgpu_fp64_selftest(int(seed), int(cases), ctypes.byref(m), ctypes.byref(d)))
     return m.value, d.value
+
+
+def arith_selftest(cases=1 << 24, seed=1):
+    """Mismatches against the FP64 unit of the square root, the quotients by a shared divisor, the
+    grouped products, quotients and roots, the equal-operand sum and the FP32 product-difference."""
+    bad = (ctypes.c_longlong * 5)()
+    check(lib().hgpu_arith_selftest(int(seed), int(cases), bad))
+    return dict(zip(("root", "shared_divisor", "groups", "equal_sum", "float_difference"), bad))
 
 
 def limiter_selftest(cases=1 << 26, seed=1):

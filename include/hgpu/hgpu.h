@@ -446,6 +446,13 @@ int hgpu_fp64_peak(double* fma_per_second);
  * of differing results (NaN == NaN). */
 int hgpu_fp64_selftest(unsigned long long seed, long long cases, long long* mul_mismatches,
                        long long* div_mismatches);
+/* Self-test of the kernels' other replacements for the FP64 unit: the integer-pipe square
+ * root; quotients by a shared divisor, its reciprocal formed on the device or the host;
+ * the products, quotients and roots of operands tested as a group; the sum of two equal
+ * numbers; and the FP32 flux's c - a b, rounded as through binary64 (operands beside
+ * midpoints of two floats among them).  Compares each with the FP64 unit, bit for bit, on
+ * `cases` seeded operands and returns the five counts of differing results. */
+int hgpu_arith_selftest(unsigned long long seed, long long cases, long long mismatches[5]);
 /* Self-test of the kernels' bit-pattern MinMod and Superbee (FP64): compares them with
  * the res/SlopeLimiter.cl expressions under C-library fmin/fmax semantics, bit for bit
  * (signs of zero included), on `cases` seeded ratios; returns the mismatch count. */
