@@ -412,8 +412,10 @@ struct CheckedOps {
 // one fma rounds it to 24 directly, the same unless the 53-bit value is the midpoint of
 // two floats.  The distance x - r of the exact value from the fma's result r is formed
 // from the product's and the sum's error terms (fma residual, Knuth's two-sum) to well
-// below 2^-18 of half an ulp; results within that of a midpoint (and r a power of two,
-// whose lower neighbour is closer, and tiny r) take the double expression out of line.
+// below 2^-18 of half an ulp; results within that of a midpoint, or with error terms that
+// are not numbers (a product past the floats beside a c that brings the result back: the
+// comparison is false for NaN), and r a power of two, whose lower neighbour is closer, and
+// tiny r, take the double expression out of line.
 // The three conversions to double, the product, the difference and the conversion back
 // ran on the FP64 unit and were most of the FP32 flux kernel: KH 2048^2 550 us a launch,
 // 163 us with this form (the rest of it: loads at the HBM rate).
@@ -428,7 +430,7 @@ __device__ __forceinline__ float subProduct(float c, float a, float b) {
     const float e = __fsub_rn(__fadd_rn(__fsub_rn(s, r), t), pe);
     const unsigned rb = __float_as_uint(r);
     const float half = __uint_as_float(rb & 0x7F800000u) * 0x1p-24f;         // half an ulp of r
-    const bool near = fabsf(fabsf(e) - half) < 0x1p-18f * (half + fabsf(pe) + fabsf(t));
+    const bool near = !(fabsf(fabsf(e) - half) >= 0x1p-18f * (half + fabsf(pe) + fabsf(t)));
     const bool edge = (rb << 1) != 0 && ((rb << 9) == 0 || (rb & 0x7FFFFFFFu) < 0x12800000u);   // |r| < 2^-90
     return near || edge ? subProductNative(c, a, b) : r;
 }

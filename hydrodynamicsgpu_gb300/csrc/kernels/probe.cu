@@ -71,15 +71,23 @@ __device__ double windowOperand(unsigned long long s) {
 __device__ __forceinline__ bool windowed(double x) { return fabs(x) >= 0x1p-480 && fabs(x) < 0x1p481; }
 
 // floats for c - a b: any bits; c beside a b; c - a b beside a midpoint of two floats, by less
-// than a double resolves; c a power of two
+// than a double resolves; c a power of two; a b = (2^25 - 1) 2^103, the midpoint between the
+// largest float and 2^128, or a huge product, beside a c of any size
 __device__ void subOperands(unsigned long long s, float& c, float& a, float& b) {
     const unsigned long long r = splitmix(s), t = splitmix(s ^ 0x51ull);
     const unsigned sc = (unsigned)(t >> 60 & 1) << 31, sa = (unsigned)(t >> 61 & 1) << 31, sb = (unsigned)(t >> 62 & 1) << 31;
-    const int cls = (int)(s % 4);
+    const int cls = (int)(s % 5);
     if (cls == 0) {
         c = __uint_as_float((unsigned)r);
         a = __uint_as_float((unsigned)(r >> 32));
         b = __uint_as_float((unsigned)t);
+        return;
+    }
+    if (cls == 4) {
+        c = __uint_as_float(sc | (1u + (unsigned)(r % 254)) << 23 | ((unsigned)(r >> 16) & 0x7FFFFFu));
+        a = __uint_as_float(sa | (unsigned)__float_as_int(18631.f * 0x1p60f));
+        b = __uint_as_float(sb | (unsigned)__float_as_int(1801.f * 0x1p43f));
+        if (t & 1) b = __uint_as_float(sb | 180u << 23 | ((unsigned)(t >> 8) & 0x7FFFFFu));
         return;
     }
     const unsigned ea = 100u + (unsigned)(r % 50), eb = 100u + (unsigned)(r >> 8) % 50;
