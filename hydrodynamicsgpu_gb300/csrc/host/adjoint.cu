@@ -87,7 +87,8 @@ void RoeAdjoint::forward(const double* u_n, double dt, Tape& t, double* u_next, 
     launchBoundary<double>(g, methods_, cur, stream_);
     launchRoeBasis<double>(g, ph_, cur, t.basis.as<double>(), 0, stream_);
     if (dtOut) {                                   // Solver::update's CFL dt
-        launchRoeDt<double>(g, ph_, t.basis.as<double>(), integ_, acc_.as<CflAcc>(), sc, stream_);
+        launchRoeDt<double>(g, ph_, t.basis.as<double>(), integ_, acc_.as<CflAcc>(), sc, health_.as<unsigned>(),
+                            stream_);
         cudaCheck(cudaMemcpyAsync(dtOut, &sc->dt_f64, sizeof(double), cudaMemcpyDeviceToDevice, stream_), "record dt");
     } else {
         launchFixedDt<double>(ph_, integ_, dt, sc, stream_);

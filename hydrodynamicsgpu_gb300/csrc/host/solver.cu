@@ -864,7 +864,7 @@ template <typename real>
 void Roe<real>::cflReduce() {
     this->launch("cfl_min_reduce", 1, [&] {
         launchRoeDt<real>(this->rc.grid, this->ph, basis.template as<real>(), this->rc.cfg.integrator,
-                          this->dtAcc.template as<CflAcc>(), this->sc(), this->stream);
+                          this->dtAcc.template as<CflAcc>(), this->sc(), this->health, this->stream);
     });
 }
 
@@ -1006,7 +1006,7 @@ bool Roe<real>::smallStep() {
     real* next = fe ? this->flux.template as<real>() : state;      // the flux buffer is free: the fluxes stay on chip
     this->launch("roe_prologue", 1, [&] {
         launchSmallPrologue<real>(g, this->ph, this->methods, state, basis.template as<real>(), this->rc.cfg.integrator,
-                                  this->dtAcc.template as<CflAcc>(), this->sc(), this->stream);
+                                  this->dtAcc.template as<CflAcc>(), this->sc(), this->health, this->stream);
     });
     this->integrator->integrateSmall([&](const CombinePlan<real>& plan) {
         this->launch("roe_stage", 1, [&] {
@@ -1059,7 +1059,7 @@ template <typename real>
 void HLL<real>::calcTimestep() {                             // HLL::calcTimestep (HLL.cpp:35-38)
     this->launch("cfl_min_reduce", 1, [&] {
         launchHllcDt<real>(this->rc.grid, this->ph, waves.template as<real>(), this->rc.cfg.integrator,
-                           this->dtAcc.template as<CflAcc>(), this->sc(), this->stream);
+                           this->dtAcc.template as<CflAcc>(), this->sc(), this->health, this->stream);
     });
 }
 

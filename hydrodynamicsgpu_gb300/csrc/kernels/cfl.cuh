@@ -41,10 +41,12 @@ __device__ __forceinline__ void blockMaxSpeeds(unsigned long long (&s)[D], CflAc
 // The end of a CFL kernel, all threads of the block: the last block of the grid turns the
 // maxima into dt = cfl * min (starting from accInit, the bits of the largest value the
 // reference's buffer can hold) and the step's constants.  ROE: dx / (speed + 1e-9) in
-// double, else dx / speed.
+// double, else dx / speed.  A speed is never NaN and dx is positive, so a cell's quotient is
+// NaN where both are infinite, and then that of the axis's largest speed is too: it sets the
+// health bit.
 template <typename real, int D, bool ROE>
 __device__ __forceinline__ void finishCfl(const Phys<real>& ph, int integ, unsigned long long accInit, CflAcc* acc,
-                                          StepConst<real>* sc) {
+                                          StepConst<real>* sc, unsigned* health) {
     __shared__ bool last;
     __threadfence();
     __syncthreads();
@@ -53,13 +55,16 @@ __device__ __forceinline__ void finishCfl(const Phys<real>& ph, int integ, unsig
     if (!last) return;
     __threadfence();
     unsigned long long best = accInit;
+    bool nan = false;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
         const unsigned long long b = __ldcg(&acc->speed[a]);
         const real speed = (real)bitsToDouble(b, sizeof(real) == 4);
         const real q = ROE ? (real)divI((double)ph.dx[a], (double)speed + 1e-9) : divI(ph.dx[a], speed);
         best = realBits(q) < best ? realBits(q) : best;
+        nan |= isNaNBits(q);
     }
+    if (nan && threadIdx.x == 0) atomicOr(health, HEALTH_NONFINITE_DT);
     const real dt = (real)((real)bitsToDouble(best, sizeof(real) == 4) * (real)ph.cfl);   // Solver.cpp:515
     __syncthreads();                                       // every thread has read the maxima
     for (int i = threadIdx.x; i < 24; i += blockDim.x) {

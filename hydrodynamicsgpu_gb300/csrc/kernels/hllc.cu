@@ -43,7 +43,8 @@ inline unsigned cflBlocks(long long n) { return std::min(blocksFor(n), 152u * 8u
 
 template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) hllcDtKernel(Grid g, Phys<real> ph, const real* waves, int integ,
-                                                        unsigned long long accInit, CflAcc* acc, StepConst<real>* sc) {
+                                                        unsigned long long accInit, CflAcc* acc, StepConst<real>* sc,
+                                                        unsigned* health) {
     dependentLaunch();
     unsigned long long s[D] = {};
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < g.V;
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(kThreads) hllcDtKernel(Grid g, Phys<real> ph, 
         }
     }
     blockMaxSpeeds<D>(s, acc);
-    finishCfl<real, D, false>(ph, integ, accInit, acc, sc);
+    finishCfl<real, D, false>(ph, integ, accInit, acc, sc, health);
 }
 
 template <typename real, int D, bool HLL, bool GRAV>
@@ -175,16 +176,16 @@ void launchHllcWaves(const Grid& g, const Phys<real>& ph, const real* state, rea
 
 template <typename real>
 void launchHllcDt(const Grid& g, const Phys<real>& ph, const real* waves, int integrator, CflAcc* acc,
-                 StepConst<real>* sc, cudaStream_t st) {
+                 StepConst<real>* sc, unsigned* health, cudaStream_t st) {
     // the first V entries of the reference's buffer are written; with dim > 1 the rest keep
     // their initial max() (Solver.cpp:217-222, EulerHLLC.cl:135-168) and join the minimum
     const real top = g.dim > 1 ? std::numeric_limits<real>::max() : std::numeric_limits<real>::infinity();
     unsigned long long accInit = 0;
     std::memcpy(&accInit, &top, sizeof top);
     const unsigned b = cflBlocks(g.V);
-    if (g.dim == 1) launchDependent(hllcDtKernel<real, 1>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc);
-    else if (g.dim == 2) launchDependent(hllcDtKernel<real, 2>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc);
-    else launchDependent(hllcDtKernel<real, 3>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc);
+    if (g.dim == 1) launchDependent(hllcDtKernel<real, 1>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc, health);
+    else if (g.dim == 2) launchDependent(hllcDtKernel<real, 2>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc, health);
+    else launchDependent(hllcDtKernel<real, 3>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc, health);
 }
 
 template <typename real, bool GRAV>
@@ -241,7 +242,7 @@ void launchHllcFlux(const Grid& g, const Phys<real>& ph, const real* stage, cons
     template void launchHllcWaves<real>(const Grid&, const Phys<real>&, const real*, real*, int, cudaStream_t,    \
                                         const real*, long long, long long);                                       \
     template void launchHllcDt<real>(const Grid&, const Phys<real>&, const real*, int, CflAcc*, StepConst<real>*, \
-                                     cudaStream_t);                                                               \
+                                     unsigned*, cudaStream_t);                                                     \
     template void launchHllcFlux<real>(const Grid&, const Phys<real>&, const real*, const real*, real*, unsigned*, \
                                        int, cudaStream_t, const real*, long long, long long);
 INST(double)

@@ -47,7 +47,7 @@ void launchBoundary(const Grid& g, const int methods[3][2], real* state, cudaStr
 struct CflAcc;
 template <typename real>
 void launchSmallPrologue(const Grid& g, const Phys<real>& ph, const int methods[3][2], real* state, real* basis,
-                         int integrator, CflAcc* acc, StepConst<real>* sc, cudaStream_t st);
+                         int integrator, CflAcc* acc, StepConst<real>* sc, unsigned* health, cudaStream_t st);
 template <typename real>
 void launchSmallStage(const Grid& g, const Phys<real>& ph, int limiter, const StepConst<real>* sc, const real* basis,
                       const CombinePlan<real>& plan, cudaStream_t st);
@@ -91,7 +91,7 @@ int roeBasisSlowTile(int dim);
 template <typename real>
 // the step's CFL timestep and constants into sc (acc: zero before and after)
 void launchRoeDt(const Grid& g, const Phys<real>& ph, const real* basis, int integrator, CflAcc* acc,
-                 StepConst<real>* sc, cudaStream_t st);
+                 StepConst<real>* sc, unsigned* health, cudaStream_t st);
 template <typename real>
 // cells [c0, c1) only (c1 < 0: to the end of the grid)
 void launchRoeDeltaQ(const Grid& g, const real* stage, const real* basis, real* dq, int seam, cudaStream_t st,
@@ -109,7 +109,7 @@ void launchHllcWaves(const Grid& g, const Phys<real>& ph, const real* state, rea
                      const real* pot = nullptr, long long c0 = 0, long long c1 = -1);
 template <typename real>
 void launchHllcDt(const Grid& g, const Phys<real>& ph, const real* waves, int integrator, CflAcc* acc,
-                  StepConst<real>* sc, cudaStream_t st);
+                  StepConst<real>* sc, unsigned* health, cudaStream_t st);
 template <typename real>
 void launchHllcFlux(const Grid& g, const Phys<real>& ph, const real* stage, const real* waves, real* flux,
                     unsigned* health, int hll, cudaStream_t st, const real* pot = nullptr, long long c0 = 0,

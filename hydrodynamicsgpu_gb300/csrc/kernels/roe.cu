@@ -63,7 +63,8 @@ inline unsigned cflBlocks(long long n) { return std::min(blocksFor(n), 152u * 8u
 
 template <typename real, int D>
 __global__ void __launch_bounds__(kThreads) roeDtKernel(Grid g, Phys<real> ph, const real* basis, int integ,
-                                                        unsigned long long accInit, CflAcc* acc, StepConst<real>* sc) {
+                                                        unsigned long long accInit, CflAcc* acc, StepConst<real>* sc,
+                                                        unsigned* health) {
     dependentLaunch();
     unsigned long long s[D] = {};
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < g.V;
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(kThreads) roeDtKernel(Grid g, Phys<real> ph, c
         }
     }
     blockMaxSpeeds<D>(s, acc);
-    finishCfl<real, D, true>(ph, integ, accInit, acc, sc);
+    finishCfl<real, D, true>(ph, integ, accInit, acc, sc, health);
 }
 
 template <typename real, int D>
@@ -173,14 +174,14 @@ int roeBasisSlowTile(int dim) { return dim == 2 ? BasisTile<2>::Y : dim == 3 ? B
 
 template <typename real>
 void launchRoeDt(const Grid& g, const Phys<real>& ph, const real* basis, int integrator, CflAcc* acc,
-                 StepConst<real>* sc, cudaStream_t st) {
+                 StepConst<real>* sc, unsigned* health, cudaStream_t st) {
     const real top = std::numeric_limits<real>::infinity();   // outside the interior the reference's buffer holds INFINITY
     unsigned long long accInit = 0;
     std::memcpy(&accInit, &top, sizeof top);
     const unsigned b = cflBlocks(g.V);
-    if (g.dim == 1) launchDependent(roeDtKernel<real, 1>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc);
-    else if (g.dim == 2) launchDependent(roeDtKernel<real, 2>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc);
-    else launchDependent(roeDtKernel<real, 3>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc);
+    if (g.dim == 1) launchDependent(roeDtKernel<real, 1>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc, health);
+    else if (g.dim == 2) launchDependent(roeDtKernel<real, 2>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc, health);
+    else launchDependent(roeDtKernel<real, 3>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc, health);
 }
 
 // cells [c0, c1) (c1 < 0: to the end of the grid); whole-grid launches take every cell
@@ -254,7 +255,7 @@ void launchRoeFlux(const Grid& g, int limiter, const real* stage, const real* ba
     template void launchRoeBasis<real>(const Grid&, const Phys<real>&, const real*, real*, int, cudaStream_t,    \
                                        const real*, int, int);                                                  \
     template void launchRoeDt<real>(const Grid&, const Phys<real>&, const real*, int, CflAcc*, StepConst<real>*, \
-                                    cudaStream_t);                                                             \
+                                    unsigned*, cudaStream_t);                                                  \
     template void launchRoeDeltaQ<real>(const Grid&, const real*, const real*, real*, int, cudaStream_t,        \
                                         long long, long long);                                                  \
     template void launchRoeFlux<real>(const Grid&, int, const real*, const real*, const real*,                   \

@@ -48,7 +48,8 @@ template <typename real, int D>
 __global__ void __launch_bounds__(SmallTile<D>::THREADS) smallPrologueKernel(Grid g, Phys<real> ph, Methods bc,
                                                                           real* state, real* __restrict__ basis,
                                                                           int integ, unsigned long long accInit,
-                                                                          CflAcc* acc, StepConst<real>* sc) {
+                                                                          CflAcc* acc, StepConst<real>* sc,
+                                                                          unsigned* health) {
     dependentLaunch();
     typedef SmallTile<D> T;
     typedef RoeRec<D> R_;
@@ -109,7 +110,7 @@ __global__ void __launch_bounds__(SmallTile<D>::THREADS) smallPrologueKernel(Gri
         }
     }
     blockMaxSpeeds<D>(s, acc);
-    finishCfl<real, D, true>(ph, integ, accInit, acc, sc);
+    finishCfl<real, D, true>(ph, integ, accInit, acc, sc, health);
 }
 
 template <typename real, int D, int LIM, bool POST>
@@ -250,7 +251,7 @@ void smallStageLim(const Grid& g, const Phys<real>& ph, int lim, const StepConst
 
 template <typename real>
 void launchSmallPrologue(const Grid& g, const Phys<real>& ph, const int methods[3][2], real* state, real* basis,
-                         int integrator, CflAcc* acc, StepConst<real>* sc, cudaStream_t st) {
+                         int integrator, CflAcc* acc, StepConst<real>* sc, unsigned* health, cudaStream_t st) {
     const real top = std::numeric_limits<real>::infinity();
     unsigned long long accInit = 0;
     std::memcpy(&accInit, &top, sizeof top);
@@ -258,10 +259,10 @@ void launchSmallPrologue(const Grid& g, const Phys<real>& ph, const int methods[
     std::memcpy(bc.m, methods, sizeof bc.m);
     if (g.dim == 1)
         launchDependent(smallPrologueKernel<real, 1>, smallGridOf<1>(g), SmallTile<1>::THREADS, 0, st, g, ph, bc, state,
-                        basis, integrator, accInit, acc, sc);
+                        basis, integrator, accInit, acc, sc, health);
     else
         launchDependent(smallPrologueKernel<real, 2>, smallGridOf<2>(g), SmallTile<2>::THREADS, 0, st, g, ph, bc, state,
-                        basis, integrator, accInit, acc, sc);
+                        basis, integrator, accInit, acc, sc, health);
 }
 
 template <typename real>
@@ -292,7 +293,7 @@ void launchSmallFinish(const Grid& g, const int methods[3][2], const real* next,
 
 #define INST(real)                                                                                                   \
     template void launchSmallPrologue<real>(const Grid&, const Phys<real>&, const int[3][2], real*, real*, int,      \
-                                            CflAcc*, StepConst<real>*, cudaStream_t);                                \
+                                            CflAcc*, StepConst<real>*, unsigned*, cudaStream_t);                     \
     template void launchSmallStage<real>(const Grid&, const Phys<real>&, int, const StepConst<real>*, const real*,   \
                                          const CombinePlan<real>&, cudaStream_t);                                    \
     template void launchSmallFinish<real>(const Grid&, const int[3][2], const real*, real*, const StepConst<real>*,  \

@@ -244,7 +244,7 @@ int hgpu_synchronize(hgpu_solver* s);
 /* ---- failure detection.  The reference has none (it only throws at set-up:
  *      src/Solver/Solver.cpp:150-153, 201); here every step ends, and every upload
  *      is followed, by a check of the state's interior cells on the device. ---- */
-#define HGPU_HEALTH_NONFINITE_DT    1u   /* a NaN in the CFL reduction                            */
+#define HGPU_HEALTH_NONFINITE_DT    1u   /* a NaN in the CFL reduction: infinite dx and wave speed  */
 #define HGPU_HEALTH_HLLC_NOBRANCH   2u   /* an HLLC interface where no flux branch was taken       */
 #define HGPU_HEALTH_STATE_NONFINITE 4u   /* a NaN or infinity in a checked state                   */
 #define HGPU_HEALTH_STATE_DENSITY   8u   /* density <= 0 in a checked state                        */
