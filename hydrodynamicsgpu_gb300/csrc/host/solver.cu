@@ -981,11 +981,12 @@ int Roe<real>::setFusedStages(bool on) {
 // The grids that run as roe_small.cu's few launches: 1D, and 2D where the fused stage is
 // not offered (ForwardEuler or FP32: a 2D FP64 Runge-Kutta stage stays the four kernels that
 // hgpu_set_fused_stages replaces by two), up to the size where the recomputed faces cost
-// more than the launches.  us a step, this path / the kernels for large grids: 1D RK2
-// Superbee FP64 1028 cells 28 / 39, 65536 43 / 66 (FP32 16 / 25, 21 / 29); 2D ForwardEuler
-// FP64 64^2 31 / 55, 181^2 56 / 60; 2D RK2 FP32 64^2 19 / 33, 256^2 33 / 39.  Past the lines,
-// when the path was made: 1D 2^20 446 / 434 (FP32 262144 45 / 42), ForwardEuler 256^2
-// 108 / 86, FP32 512^2 76 / 61.
+// more than the launches.  us a step, this path / the kernels for large grids:
+//   1D RK2 Superbee FP64  65536 41 / 63, 200000 81 / 88, 262144 97 / 103, 2^20 446 / 434
+//                   FP32  65536 19 / 27, 200000 33 / 35, 230000 35 / 35, 262144 39 / 39
+//   2D ForwardEuler FP64  128^2 35 / 59, 181^2 55 / 62, 200^2 60 / 65, 256^2 80 / 72
+//   2D RK2          FP32  200^2 27 / 35, 316^2 40 / 44, 400^2 52 / 49 (ForwardEuler 316^2 31 / 34, 400^2 39 / 37)
+// The 1D line is where FP32 stops gaining; FP64 would gain 5 % up to a little further.
 template <typename real>
 bool Roe<real>::smallGrid() const {
     const auto& c = this->rc.cfg;
