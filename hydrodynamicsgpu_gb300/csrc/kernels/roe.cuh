@@ -248,7 +248,15 @@ __device__ __forceinline__ void rightTransformDense(const real* rec, const real*
     }
 }
 
-// The rows of L x and R f (below) with a group's products.
+// The group for any operands: each product tests its own pair.
+struct GroupAny {
+    static __device__ __forceinline__ double mul(double x, double y) { return mulI(x, y); }
+    static __device__ __forceinline__ double div(double x, double y) { return divI(x, y); }
+    static __device__ __forceinline__ double half(double p) { return halfOf(p); }
+};
+
+// The rows of L x and R f (below) with a group's products, for finite x and f (common.cuh's
+// rule for zero and unit coefficients).
 template <typename G, int D, int SIDE>
 __device__ __forceinline__ void leftRows(const double* rec, const double* x, double* y) {
     typedef RoeRec<D> R_;
@@ -289,6 +297,31 @@ __device__ __forceinline__ void rightRows(const double* rec, const double* f, do
     for (int g = 0; g < N; ++g) F[g] = Fr[perm<SIDE>(g)];
 }
 
+// The transforms of a warp whose operands are not all in a group's window: each product tests
+// its own pair, and operands that are not finite take the dense sums.  1D and 2D call them out
+// of line, on copies that only such a warp makes: inlined they cost the ordinary warps (1D shock
+// tube run 5.86 -> 6.11 ms; called, 5.83); 3D inlines them (96^3 step 2.40 ms either way).  A
+// step of gas whose transverse velocities are 1e-200 throughout, RungeKutta4, by these / by the
+// dense sums for every such warp: 1024^2 2.01 / 2.41 ms, 96^3 2.81 / 3.75 ms.
+template <int D, int SIDE>
+__device__ __forceinline__ void leftTransformAny(const double* rec, const double* x, double* y) {
+    if (allFinite<double, D + 2>(x)) leftRows<GroupAny, D, SIDE>(rec, x, y);
+    else leftTransformDense<double, D, SIDE>(rec, x, y);
+}
+template <int D, int SIDE>
+__device__ __forceinline__ void rightTransformAny(const double* rec, const double* f, double* F) {
+    if (allFinite<double, D + 2>(f)) rightRows<GroupAny, D, SIDE>(rec, f, F);
+    else rightTransformDense<double, D, SIDE>(rec, f, F);
+}
+template <int D, int SIDE>
+__device__ __noinline__ void leftTransformCall(const double* rec, const double* x, double* y) {
+    leftTransformAny<D, SIDE>(rec, x, y);
+}
+template <int D, int SIDE>
+__device__ __noinline__ void rightTransformCall(const double* rec, const double* f, double* F) {
+    rightTransformAny<D, SIDE>(rec, f, F);
+}
+
 // y = L x with L in the global frame: y_i = sum_j L[i][perm(j)] x_j, j ascending.
 // FLAT: the caller's x is a difference of neighbouring states, often exactly zero.
 template <typename real, int D, int SIDE, bool FLAT = false>
@@ -314,13 +347,22 @@ __device__ __forceinline__ void leftTransform(const real* rec, const real* x, re
         }
     }
     if constexpr (sizeof(real) == 8) {
-        // the record's rows and x without a zero, with zeros, or neither (common.cuh's rule
-        // for finite operands then needs the dense sums)
+        // the record's rows and x without a zero, with zeros, or neither
         if (warpAll(allInWindow<N>(x) & allInWindow<R_::NB - R_::VT>(rec + R_::VT)))
             leftRows<GroupPlain, D, SIDE>(rec, x, y);
         else if (warpAll(allInWindowOrZero<N>(x) & allInWindowOrZero<R_::NB - R_::VT>(rec + R_::VT)))
             leftRows<GroupZeros, D, SIDE>(rec, x, y);
-        else leftTransformDense<real, D, SIDE>(rec, x, y);
+        else if constexpr (D == 3) leftTransformAny<D, SIDE>(rec, x, y);
+        else {
+            double r[R_::NB], a[N], b[N];
+#pragma unroll
+            for (int k = R_::VT; k < R_::NB; ++k) r[k] = rec[k];
+#pragma unroll
+            for (int j = 0; j < N; ++j) a[j] = x[j];
+            leftTransformCall<D, SIDE>(r, a, b);
+#pragma unroll
+            for (int j = 0; j < N; ++j) y[j] = b[j];
+        }
         return;
     }
     if (!allFinite<real, N>(x)) { leftTransformDense<real, D, SIDE>(rec, x, y); return; }
@@ -361,7 +403,17 @@ __device__ __forceinline__ void rightTransform(const real* rec, const real* f, r
         if (warpAll(allInWindow<N>(f) & allInWindow<R_::L0>(rec))) rightRows<GroupPlain, D, SIDE>(rec, f, F);
         else if (warpAll(allInWindowOrZero<N>(f) & allInWindowOrZero<R_::L0>(rec)))
             rightRows<GroupZeros, D, SIDE>(rec, f, F);
-        else rightTransformDense<real, D, SIDE>(rec, f, F);
+        else if constexpr (D == 3) rightTransformAny<D, SIDE>(rec, f, F);
+        else {
+            double r[R_::L0], a[N], b[N];
+#pragma unroll
+            for (int k = 0; k < R_::L0; ++k) r[k] = rec[k];
+#pragma unroll
+            for (int j = 0; j < N; ++j) a[j] = f[j];
+            rightTransformCall<D, SIDE>(r, a, b);
+#pragma unroll
+            for (int j = 0; j < N; ++j) F[j] = b[j];
+        }
         return;
     }
     if (!allFinite<real, N>(f)) { rightTransformDense<real, D, SIDE>(rec, f, F); return; }
@@ -458,11 +510,6 @@ __device__ __forceinline__ void roeFlux(const real* rec, const real* sL, const r
 // Each pass keeps far fewer values live than the fused form, so more warps fit per SM.
 // REC also stores the per-wave tape values of this pass (A, phi, phi', r; the caller
 // offsets tape to the face, as for roeFlux).
-struct GroupAny {
-    static __device__ __forceinline__ double mul(double x, double y) { return mulI(x, y); }
-    static __device__ __forceinline__ double div(double x, double y) { return divI(x, y); }
-    static __device__ __forceinline__ double half(double p) { return halfOf(p); }
-};
 template <typename G, int D, int SIDE, int LIM, bool REC>
 __device__ __forceinline__ void correctionsOf(const double* rec, const double* upwind, const double* dq, double dt_dx,
                                               int lim, double* corr, double* __restrict__ tape, long long V) {
