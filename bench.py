@@ -553,9 +553,10 @@ def adjoint_measure(hg, _abi, ic, args):
 # same kernels on KH 1024x1024 (dram__bytes_read.sum + dram__bytes_write.sum over the
 # interior cells); traffic grows with the cells processed, so the bench workload's
 # per-launch traffic is this times its interior cells.  roe_flux is its two passes
-# together (corrections 148 B + transforms 420 B).
-MEASURED_TRAFFIC_PER_CELL = {"roe_flux": 568.0, "roe_delta_q_tilde": 252.0, "roe_eigenbasis": 245.0,
-                             "flux_divergence_combine": 123.0}
+# together (corrections 146 B + transforms 418 B); the combine's is the mean of stages 1, 2
+# and 4 (120, 193 and 142 B).
+MEASURED_TRAFFIC_PER_CELL = {"roe_flux": 563.7, "roe_delta_q_tilde": 249.7, "roe_eigenbasis": 247.6,
+                             "flux_divergence_combine": 151.6}
 
 # Instructions the FP64 unit executes per interior cell of one launch of each kernel of
 # the EulerRoe FP64 step (MinMod), from ncu's smsp__inst_executed_pipe_fp64 (warp

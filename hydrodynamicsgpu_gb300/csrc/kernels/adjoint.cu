@@ -475,7 +475,8 @@ __global__ void adjBoundaryKernel(Grid g, int axis, int N, int mMin, int mMax, d
 void launchAdjFlux(const Grid& g, const Phys<double>& ph, int limiter, const double* dtdx, const double* stage,
                    const double* dq, const double* basis, const double* fluxTape, const AdjStage& st,
                    const AdjScratch& s, int first, cudaStream_t stream) {
-#define L(DD) launchDependent(adjFluxKernel<DD>, blocksFor(g.V), kT, 0, stream, g, ph, limiter, dtdx[0], dtdx[1], dtdx[2], stage, dq, basis, fluxTape, st, s, first)
+#define L(DD) launchDependent(adjFluxKernel<DD>, blocksFor(g.V), kT, 0, stream, g, ph, limiter, dtdx[0], dtdx[1], \
+        dtdx[2], stage, dq, basis, fluxTape, st, s, first)
     if (g.dim == 1) { L(1); }
     else if (g.dim == 2) { L(2); }
     else { L(3); }
@@ -521,7 +522,8 @@ void launchAdjBoundary(const Grid& g, const int methods[3][2], double* lam, cuda
     for (int axis = g.dim - 1; axis >= 0; --axis) {
         int A = axis == 0 ? 1 : 0, B = axis == 2 ? 1 : 2;
         long long lines = g.dim == 1 ? 1 : (long long)g.S[A] * g.S[B];
-        launchDependent(adjBoundaryKernel, blocksFor(lines), kT, 0, stream, g, axis, g.dim + 2, methods[axis][0], methods[axis][1],
+        launchDependent(adjBoundaryKernel, blocksFor(lines), kT, 0, stream, g, axis, g.dim + 2, methods[axis][0],
+                methods[axis][1],
                                                                lam);
     }
 }

@@ -224,9 +224,12 @@ __global__ void __launch_bounds__(256) batchWaveKernel(const BatchProblem<real>*
 
 template <typename real>
 void BatchLaunch<real>::boundary(unsigned* q) const {
-    if (dim == 1) launchDependent(batchBoundaryKernel<real, 1>, persistentBlocks(batchBoundaryKernel<real, 1>, 0, tu.blocksPerSM, nP), 256, 0, st, P, nP, state, q);
-    else if (dim == 2) launchDependent(batchBoundaryKernel<real, 2>, persistentBlocks(batchBoundaryKernel<real, 2>, 0, tu.blocksPerSM, nP), 256, 0, st, P, nP, state, q);
-    else launchDependent(batchBoundaryKernel<real, 3>, persistentBlocks(batchBoundaryKernel<real, 3>, 0, tu.blocksPerSM, nP), 256, 0, st, P, nP, state, q);
+    if (dim == 1) launchDependent(batchBoundaryKernel<real, 1>,
+            persistentBlocks(batchBoundaryKernel<real, 1>, 0, tu.blocksPerSM, nP), 256, 0, st, P, nP, state, q);
+    else if (dim == 2) launchDependent(batchBoundaryKernel<real, 2>,
+            persistentBlocks(batchBoundaryKernel<real, 2>, 0, tu.blocksPerSM, nP), 256, 0, st, P, nP, state, q);
+    else launchDependent(batchBoundaryKernel<real, 3>,
+            persistentBlocks(batchBoundaryKernel<real, 3>, 0, tu.blocksPerSM, nP), 256, 0, st, P, nP, state, q);
 }
 
 template <typename real>
@@ -243,7 +246,8 @@ void BatchLaunch<real>::roeBasis(int loA, int hiA, unsigned* q) const {
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                                        \
         launchDependent(batchRoeBasisKernel<real, DD, true>, nT, 256, smem, st, P, tiles, nT, tu, loA, hiA, state, faces, q);    \
     else                                                                                                           \
-        launchDependent(batchRoeBasisKernel<real, DD, false>, persistentBlocks(batchRoeBasisKernel<real, DD, false>, smem, tu.blocksPerSM, nT), 256, smem, st,               \
+        launchDependent(batchRoeBasisKernel<real, DD, false>, \
+                persistentBlocks(batchRoeBasisKernel<real, DD, false>, smem, tu.blocksPerSM, nT), 256, smem, st, \
             P, tiles, nT, tu, loA, hiA, state, faces, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }
@@ -253,7 +257,9 @@ void BatchLaunch<real>::roeBasis(int loA, int hiA, unsigned* q) const {
 
 template <typename real>
 void BatchLaunch<real>::waves(int hll, unsigned* q) const {
-#define L(DD, H) launchDependent(batchWaveKernel<real, DD, H>, persistentBlocks(batchWaveKernel<real, DD, H>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, state, faces, q)
+#define L(DD, H) launchDependent(batchWaveKernel<real, DD, H>, \
+        persistentBlocks(batchWaveKernel<real, DD, H>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, \
+        state, faces, q)
     if (hll) {
         if (dim == 1) L(1, true);
         else if (dim == 2) L(2, true);
@@ -272,7 +278,9 @@ void BatchLaunch<real>::dt(int hllc, unsigned long long* acc, unsigned* health, 
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                         \
         launchDependent(batchDtKernel<real, DD, true>, nT, 256, 0, st, P, tiles, nT, tu, hllc, faces, acc, health, q);           \
     else                                                                                                           \
-        launchDependent(batchDtKernel<real, DD, false>, persistentBlocks(batchDtKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, hllc, faces, acc, health, q)
+        launchDependent(batchDtKernel<real, DD, false>, \
+                persistentBlocks(batchDtKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, \
+                nT, tu, hllc, faces, acc, health, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }
     else { L(3); }
@@ -290,7 +298,9 @@ void BatchLaunch<real>::deltaQ(int loA, int hiA, const real* stage, real* dq, un
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                                        \
         launchDependent(batchDeltaQKernel<real, DD, true>, nT, 256, 0, st, P, tiles, nT, tu, loA, hiA, stage, faces, dq, q);     \
     else                                                                                                           \
-        launchDependent(batchDeltaQKernel<real, DD, false>, persistentBlocks(batchDeltaQKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, loA, hiA, stage,  \
+        launchDependent(batchDeltaQKernel<real, DD, false>, \
+                persistentBlocks(batchDeltaQKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, \
+                tiles, nT, tu, loA, hiA, stage, \
                                                                                  faces, dq, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }
@@ -305,7 +315,9 @@ void BatchLaunch<real>::combine(const real* fluxBuf, const CombinePlan<real>& pl
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                                        \
         launchDependent(batchCombineKernel<real, DD, true>, nT, 256, 0, st, P, tiles, nT, tu, fluxBuf, plan, sc, q);             \
     else                                                                                                           \
-        launchDependent(batchCombineKernel<real, DD, false>, persistentBlocks(batchCombineKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu,  \
+        launchDependent(batchCombineKernel<real, DD, false>, \
+                persistentBlocks(batchCombineKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, \
+                tiles, nT, tu, \
                                                                                                   fluxBuf, plan, sc, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }
@@ -315,7 +327,9 @@ void BatchLaunch<real>::combine(const real* fluxBuf, const CombinePlan<real>& pl
 
 template <typename real>
 void BatchLaunch<real>::gravity(int integ, const StepConst<real>* sc, unsigned* q) const {
-#define L(DD) launchDependent(batchGravityKernel<real, DD>, persistentBlocks(batchGravityKernel<real, DD>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, integ, sc, state, q)
+#define L(DD) launchDependent(batchGravityKernel<real, DD>, \
+        persistentBlocks(batchGravityKernel<real, DD>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, \
+        integ, sc, state, q)
     if (dim == 1) L(1);
     else if (dim == 2) L(2);
     else L(3);
@@ -328,7 +342,8 @@ void BatchLaunch<real>::stateCheck(unsigned* health, unsigned* healthP, unsigned
     if (tu.blocksPerSM < 0 && tu.cpt == 1)                                                                         \
         launchDependent(batchStateCheckKernel<real, DD, true>, nT, 256, 0, st, P, tiles, nT, tu, state, health, healthP, q);     \
     else                                                                                                           \
-        launchDependent(batchStateCheckKernel<real, DD, false>, persistentBlocks(batchStateCheckKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st,                \
+        launchDependent(batchStateCheckKernel<real, DD, false>, \
+                persistentBlocks(batchStateCheckKernel<real, DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, \
             P, tiles, nT, tu, state, health, healthP, q)
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }

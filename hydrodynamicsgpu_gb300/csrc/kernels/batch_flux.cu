@@ -96,7 +96,9 @@ template <typename real, int HLLC, int LIM>
 static void batchFluxLaunch(const BatchLaunch<real>& b, int hllc, int lim, const StepConst<real>* sc,
                             const real* stage, const real* dq, real* fluxBuf, unsigned* health, unsigned* q) {
 #define L(DD)                                                                                                       \
-    launchDependent(batchFluxKernel<real, DD, HLLC, LIM>, persistentBlocks(batchFluxKernel<real, DD, HLLC, LIM>, 0, b.tu.blocksPerSM, b.nT), 256, 0, b.st, b.P, b.tiles, b.nT, b.tu, hllc, lim, sc, stage, b.faces, dq, \
+    launchDependent(batchFluxKernel<real, DD, HLLC, LIM>, \
+            persistentBlocks(batchFluxKernel<real, DD, HLLC, LIM>, 0, b.tu.blocksPerSM, b.nT), 256, 0, b.st, b.P, \
+            b.tiles, b.nT, b.tu, hllc, lim, sc, stage, b.faces, dq, \
                                                            fluxBuf, health, q)
     if (b.dim == 1) L(1);
     else if (b.dim == 2) L(2);
@@ -124,12 +126,17 @@ static void batchFluxSplitLaunch(const BatchProblem<double>* P, const BatchTile*
                                  const double* stage, const double* dq, double* fluxBuf, unsigned* q0, unsigned* q1) {
 #define L(DD)                                                                                                       \
     if (tu.blocksPerSM < 0 && tu.cpt == 1) {                                                                                       \
-        launchDependent(batchFluxCorrKernel<DD, LIM, true>, nT, 256, 0, st, P, tiles, nT, tu, lim, sc, faces, dq, fluxBuf, q0);   \
-        launchDependent(batchFluxXformKernel<DD, true>, nT, 256, 0, st, P, tiles, nT, tu, stage, faces, fluxBuf, q1);             \
+        launchDependent(batchFluxCorrKernel<DD, LIM, true>, nT, 256, 0, st, P, tiles, nT, tu, lim, sc, faces, dq, \
+                fluxBuf, q0); \
+        launchDependent(batchFluxXformKernel<DD, true>, nT, 256, 0, st, P, tiles, nT, tu, stage, faces, fluxBuf, \
+                q1); \
     } else {                                                                                                        \
-        launchDependent(batchFluxCorrKernel<DD, LIM, false>, persistentBlocks(batchFluxCorrKernel<DD, LIM, false>, 0, tu.blocksPerSM, nT), 256, 0, st,                   \
+        launchDependent(batchFluxCorrKernel<DD, LIM, false>, \
+                persistentBlocks(batchFluxCorrKernel<DD, LIM, false>, 0, tu.blocksPerSM, nT), 256, 0, st, \
             P, tiles, nT, tu, lim, sc, faces, dq, fluxBuf, q0);                                                     \
-        launchDependent(batchFluxXformKernel<DD, false>, persistentBlocks(batchFluxXformKernel<DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, nT, tu, stage, faces, fluxBuf, q1);               \
+        launchDependent(batchFluxXformKernel<DD, false>, \
+                persistentBlocks(batchFluxXformKernel<DD, false>, 0, tu.blocksPerSM, nT), 256, 0, st, P, tiles, \
+                nT, tu, stage, faces, fluxBuf, q1); \
     }
     if (dim == 1) { L(1); }
     else if (dim == 2) { L(2); }

@@ -170,9 +170,9 @@ __device__ __forceinline__ void quotientsBy(const float* df, const Divisor<float
 // Flux divergence and Runge-Kutta combine of one cell (res/CalcFluxDeriv.cl:7-44 and
 // the multAdd chain).  `off` is the cell offset of this grid inside the slot arrays
 // (0 for a single problem; the problem's first cell in a batch).
-// deltaFlux / dx with dx's reciprocal bits from the host (quotBy): KH 2048^2 FP64 237 us
-// a launch, 286 us with the x quotients by Markstein's two FMAs on the FP64 unit and the
-// rest by divI.
+// deltaFlux / dx with dx's reciprocal bits from the host (quotBy): KH 2048^2 FP64 286 -> 237 us
+// a launch against the x quotients by Markstein's two FMAs on the FP64 unit and the rest by
+// divI; 216 us with the differences loaded together (below).
 template <typename real, int D, bool FLATD = false, bool POST = false>
 __device__ __forceinline__ void derivCombineCell(const Grid& g, const Phys<real>& ph, const real* __restrict__ flux,
                                                  const CombinePlan<real>& plan, const StepConst<real>& sc,

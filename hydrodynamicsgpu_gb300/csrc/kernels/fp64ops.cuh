@@ -229,8 +229,9 @@ __device__ __forceinline__ float divI(float x, float y) { return x / y; }
 // y += y (1 - a y^2) / 2 that keep it from below (2^-28, then 2^-57); q = floor(2^53 a y) is
 // the truncated root or one less, and the remainder, exact modulo 2^64, against q rounds it
 // to nearest (a root is never a tie).  Some 60 instructions against about ten FP64
-// operations of 64 issue slots each: KH 2048^2 eigenbasis 867 -> 525 us a launch (with roe.cuh's left rows off the FP64 unit too), HLLC wave
-// speeds at 1021x1030 154 -> 105 us, at 160x144x136 889 -> 713 us.
+// operations of 64 issue slots each: KH 2048^2 eigenbasis 867 -> 525 us a launch (with roe.cuh's
+// left rows off the FP64 unit too), HLLC wave speeds at 1021x1030 154 -> 105 us, at 160x144x136
+// 889 -> 713 us.
 __device__ __forceinline__ double rootBits(unsigned xh, unsigned xl) {
     const unsigned odd = (~xh >> 20) & 1u, mh = (xh & 0xFFFFFu) | 0x100000u;
     const unsigned ah = __funnelshift_l(xl, mh, 10 + odd), al = xl << (10 + odd);          // a 2^64

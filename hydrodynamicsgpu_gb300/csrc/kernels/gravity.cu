@@ -240,7 +240,8 @@ template <typename real>
 void launchGravityCombine(const Grid& g, const GravityConst<real>& gc, const real* stage, const real* pot,
                           const CombinePlan<real>& plan, const StepConst<real>* sc, cudaStream_t st) {
     if (g.dim == 1) launchDependent(gravityCombineKernel<real, 1>, blocksFor(g.V), kThreads, 0, st, g, gc, stage, pot, plan, sc);
-    else if (g.dim == 2) launchDependent(gravityCombineKernel<real, 2>, blocksFor(g.V), kThreads, 0, st, g, gc, stage, pot, plan, sc);
+    else if (g.dim == 2) launchDependent(gravityCombineKernel<real, 2>, blocksFor(g.V), kThreads, 0, st, g, gc,
+            stage, pot, plan, sc);
     else launchDependent(gravityCombineKernel<real, 3>, blocksFor(g.V), kThreads, 0, st, g, gc, stage, pot, plan, sc);
 }
 

@@ -142,7 +142,8 @@ void launchHllcWavesG(const Grid& g, const Phys<real>& ph, const real* state, re
     if (g.dim > 1 && c0 % plane == 0 && c1 % plane == 0) {
         const int s0 = (int)(c0 / plane), s1 = (int)(c1 / plane);
 #define T(DD, H) \
-    launchDependent(hllcWaveTileKernel<real, DD, H, GRAV>, tileGrid<DD>(g, s0, s1), kThreads, 0, st, g, ph, gq, state, waves, pot, s0, s1)
+    launchDependent(hllcWaveTileKernel<real, DD, H, GRAV>, tileGrid<DD>(g, s0, s1), kThreads, 0, st, g, ph, gq, \
+            state, waves, pot, s0, s1)
         if (hll) {
             if (g.dim == 2) T(2, true);
             else T(3, true);
@@ -183,8 +184,10 @@ void launchHllcDt(const Grid& g, const Phys<real>& ph, const real* waves, int in
     unsigned long long accInit = 0;
     std::memcpy(&accInit, &top, sizeof top);
     const unsigned b = cflBlocks(g.V);
-    if (g.dim == 1) launchDependent(hllcDtKernel<real, 1>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc, health);
-    else if (g.dim == 2) launchDependent(hllcDtKernel<real, 2>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc, health);
+    if (g.dim == 1) launchDependent(hllcDtKernel<real, 1>, b, kThreads, 0, st, g, ph, waves, integrator, accInit,
+            acc, sc, health);
+    else if (g.dim == 2) launchDependent(hllcDtKernel<real, 2>, b, kThreads, 0, st, g, ph, waves, integrator,
+            accInit, acc, sc, health);
     else launchDependent(hllcDtKernel<real, 3>, b, kThreads, 0, st, g, ph, waves, integrator, accInit, acc, sc, health);
 }
 
@@ -217,7 +220,8 @@ void launchHllcFluxG(const Grid& g, const Phys<real>& ph, const real* stage, con
         return;
     }
 #define L(DD, H)                                                                                                  \
-    launchDependent(hllcFluxKernel<real, DD, H, GRAV>, blocksFor(c1 - c0), kThreads, 0, st, g, ph, stage, waves, flux, health, pot, \
+    launchDependent(hllcFluxKernel<real, DD, H, GRAV>, blocksFor(c1 - c0), kThreads, 0, st, g, ph, stage, waves, \
+            flux, health, pot, \
                                                                              c0, c1)
     if (hll) {
         if (g.dim == 1) L(1, true);

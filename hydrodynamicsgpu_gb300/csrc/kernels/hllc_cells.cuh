@@ -446,8 +446,7 @@ __device__ __forceinline__ bool hllcFluxCell(const Grid& g, const Phys<real>& ph
     return ok;
 }
 
-// primitives of the tile's cells and of one cell below along every axis, into `prim`
-// (HX*HY*HZ entries, x fastest); the caller synchronises
+// the square roots that a staged cell's wave speeds share; none for the flux's primitives
 template <typename real, int D>
 __device__ __forceinline__ void stageRoots(Prim<real, D>&, double, bool) {}
 template <typename real, int D>
@@ -455,6 +454,8 @@ __device__ __forceinline__ void stageRoots(WavePrim<real, D>& P, double gm1, boo
     P.c = hll ? soundSpeed<true>(gm1, P) : soundSpeed<false>(gm1, P);
     P.w = hll ? sqrtI(P.density) : (real)0;
 }
+// primitives of the tile's cells and of one cell below along every axis, into `prim`
+// (HX*HY*HZ entries, x fastest); the caller synchronises
 template <typename real, int D, bool GRAV, bool HLL = false, typename P>
 __device__ __forceinline__ void stagePrims(const Grid& g, const Phys<real>& ph, const real* __restrict__ st,
                                            int x0, int y0, int z0, int HX, int HY, int HZ, P* prim,

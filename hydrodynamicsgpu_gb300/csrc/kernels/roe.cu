@@ -143,7 +143,8 @@ void launchRoeBasisG(const Grid& g, const Phys<real>& ph, const real* state, rea
                     (unsigned)((g.S[2] + tz - 1) / tz));
     };
     if (g.dim == 1) {
-        launchDependent(roeBasisKernel<real, 1, GRAV>, grid(BasisTile<1>::X, 1, 1), 256, 0, st, g, ph, state, basis, loA, hiA, pot,
+        launchDependent(roeBasisKernel<real, 1, GRAV>, grid(BasisTile<1>::X, 1, 1), 256, 0, st, g, ph, state,
+                basis, loA, hiA, pot,
                                                                                    0);
         return;
     }
@@ -180,7 +181,8 @@ void launchRoeDt(const Grid& g, const Phys<real>& ph, const real* basis, int int
     std::memcpy(&accInit, &top, sizeof top);
     const unsigned b = cflBlocks(g.V);
     if (g.dim == 1) launchDependent(roeDtKernel<real, 1>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc, health);
-    else if (g.dim == 2) launchDependent(roeDtKernel<real, 2>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc, health);
+    else if (g.dim == 2) launchDependent(roeDtKernel<real, 2>, b, kThreads, 0, st, g, ph, basis, integrator,
+            accInit, acc, sc, health);
     else launchDependent(roeDtKernel<real, 3>, b, kThreads, 0, st, g, ph, basis, integrator, accInit, acc, sc, health);
 }
 
@@ -195,7 +197,8 @@ void launchRoeDeltaQ(const Grid& g, const real* stage, const real* basis, real* 
     if (c1 <= c0) return;
     const unsigned b = stageBlocks(c1 - c0);
     if (g.dim == 1) launchDependent(roeDeltaQKernel<real, 1>, b, kStageThreads, 0, st, g, stage, basis, dq, loA, hiA, c0, c1);
-    else if (g.dim == 2) launchDependent(roeDeltaQKernel<real, 2>, b, kStageThreads, 0, st, g, stage, basis, dq, loA, hiA, c0, c1);
+    else if (g.dim == 2) launchDependent(roeDeltaQKernel<real, 2>, b, kStageThreads, 0, st, g, stage, basis, dq,
+            loA, hiA, c0, c1);
     else launchDependent(roeDeltaQKernel<real, 3>, b, kStageThreads, 0, st, g, stage, basis, dq, loA, hiA, c0, c1);
 }
 
@@ -225,8 +228,10 @@ void launchRoeFluxLim(const Grid& g, int limiter, const real* stage, const real*
         return;
     }
     const unsigned b = blocksFor(c1 - c0);
-    if (g.dim == 1) launchDependent(roeFluxKernel<real, 1, LIM>, b, kThreads, 0, st, g, limiter, stage, basis, dq, sc, flux, c0, c1);
-    else if (g.dim == 2) launchDependent(roeFluxKernel<real, 2, LIM>, b, kThreads, 0, st, g, limiter, stage, basis, dq, sc, flux, c0, c1);
+    if (g.dim == 1) launchDependent(roeFluxKernel<real, 1, LIM>, b, kThreads, 0, st, g, limiter, stage, basis,
+            dq, sc, flux, c0, c1);
+    else if (g.dim == 2) launchDependent(roeFluxKernel<real, 2, LIM>, b, kThreads, 0, st, g, limiter, stage,
+            basis, dq, sc, flux, c0, c1);
     else launchDependent(roeFluxKernel<real, 3, LIM>, b, kThreads, 0, st, g, limiter, stage, basis, dq, sc, flux, c0, c1);
 }
 
